@@ -204,6 +204,7 @@ struct QueryDev {
     i64 N;          // X / u
     i64 nc;         // candidates k <= N coprime to 6
     u64 slot_base;  // first global evaluation slot of this query
+    u64 blk_base;   // first 32-candidate block of this query
     u64 win;        // S1 window length W (a power of two; 0: no windowed S1)
     u64 win_max;    // windows w < win_max lie in the dense tier ((w+1)*W <= u_dense < 2^31)
     u64 inv_limit;  // largest tabulated S1 reciprocal 1/n
@@ -313,6 +314,17 @@ struct __align__(16) SlotDesc {
 };
 static_assert(sizeof(SlotDesc) == 96, "SlotDesc is six 16-byte words");
 constexpr u64 kSlotS1Only = 1ull << 15;
+
+// Tile groups (dr_tiles.cu): the evaluations e of a 32-candidate block of a query that
+// agree in kind and strides are summed together, one divisor range for all of them.
+// kSlotTile marks the slots that take part; the group's first slot (its leader) holds the
+// group's work, counted in units of kTileN divisors of an S1 segment or kTileM wheel
+// positions of an S2 piece over the union of the members' ranges.
+constexpr u64 kSlotTile = 1ull << 16;
+constexpr uint32_t kTileN = 128;
+constexpr uint32_t kTileM = 64;
+// y below this: one FMA rounded down gives every quotient of the tile kernel exactly
+constexpr u64 kTileMaxY = 1ull << 51;
 
 #ifdef __CUDACC__
 __device__ __forceinline__ i64 piece_mcount(i64 lo, i64 hi) {
@@ -526,21 +538,22 @@ __device__ inline void decode_eval(const QueryDev& Q, const TableView& T, i64 c,
 __device__ __forceinline__ u64 stride_code(int st) { return st == 1 ? 0u : st == 2 ? 1u : st == 6 ? 2u : 3u; }
 __device__ __forceinline__ int stride_of_code(u64 c) { return c == 0 ? 1 : c == 1 ? 2 : c == 2 ? 6 : S1_WHEEL; }
 
-// An evaluation as the sums kernel needs it, written once by the planner.
-__device__ __forceinline__ void pack_slot(const EvalDesc& d, SlotDesc* out) {
+// An evaluation as the sums kernels need it, written once by the planner, with `flags` set
+// in its bits; returns the bits.
+__device__ __forceinline__ u64 pack_slot(const EvalDesc& d, SlotDesc* out, u64 flags) {
     SlotDesc s;
-    if (d.kind == EVAL_NONE) {  // no terms: the sums kernel never reads it
+    if (d.kind == EVAL_NONE) {  // no terms
         s.y = 0;
         s.A = s.B = 0;
         for (int g = 0; g < kS1Seg; ++g) s.n0[g] = s.cnt[g] = 0;
         s.bits = 0;
         *out = s;
-        return;
+        return 0;
     }
     s.y = d.y;
     s.A = d.A;
     s.B = d.kind == EVAL_COMB2 ? d.B : 0;
-    u64 bits = (u64)d.kind | (d.coef < 0 ? 4ull : 0ull) | (d.npieces == 0 ? kSlotS1Only : 0ull);
+    u64 bits = (u64)d.kind | (d.coef < 0 ? 4ull : 0ull) | (d.npieces == 0 ? kSlotS1Only : 0ull) | flags;
     for (int g = 0; g < kS1Seg; ++g) {
         s.n0[g] = d.s1_n0[g];
         s.cnt[g] = d.s1_cnt[g];
@@ -548,6 +561,7 @@ __device__ __forceinline__ void pack_slot(const EvalDesc& d, SlotDesc* out) {
     }
     s.bits = bits;
     *out = s;
+    return bits;
 }
 
 // The planner's evaluation back from its SlotDesc: S1 segments as stored, S2
@@ -576,6 +590,66 @@ __device__ __forceinline__ void unpack_slot(const SlotDesc& s, EvalDesc& d) {
         d.nseg = kS1Seg;
     }
     eval_total(d);
+}
+
+// Whether an evaluation can be summed by the tile kernel: y < 2^51, every S1 divisor
+// tabulated and below 2^31, every j below 2^31.
+__device__ __forceinline__ bool tile_eligible(const EvalDesc& d, u64 inv_limit) {
+    if (d.kind == EVAL_NONE || d.y >= kTileMaxY || d.A >= 0x7FFFFFF0ll || d.B >= 0x7FFFFFF0ll) return false;
+    const u64 lim = min(inv_limit, (u64)0x7FFFFFF0ull);
+    for (int g = 0; g < kS1Seg; ++g)
+        if (d.s1_cnt[g] > 0 && s1_n_at(d.s1_n0[g], d.s1_stride[g], (u64)(d.s1_cnt[g] - 1)) > lim) return false;
+    return true;
+}
+
+// The bits of SlotDesc.bits that the members of a tile group have in common: the kind and
+// the stride codes (then their S1 segments lie on the same arithmetic progressions).
+constexpr u64 kTileSig = 3ull | (3ull << 3) | (3ull << 6) | (3ull << 9) | (3ull << 12);
+
+// Range [lo, hi] of segment g of a tile slot (lo > hi: empty), in the units the tile kernel
+// counts: S1 segments (g < kS1Seg) by i with n = stride*i + *res (the wheel: n =
+// candidate_k(i)), S2 pieces by wheel position, with the piece's j range in jr.
+__device__ __forceinline__ void tile_range(const SlotDesc& t, int g, uint32_t* lo, uint32_t* hi, uint32_t* res,
+                                           uint2* jr) {
+    *lo = 1;
+    *hi = 0;
+    *res = 0;
+    *jr = make_uint2(1u, 0u);
+    if (g < kS1Seg) {
+        const uint32_t cnt = (uint32_t)t.cnt[g];
+        if (cnt == 0) return;
+        const uint32_t n0 = (uint32_t)t.n0[g];
+        const uint32_t code = (uint32_t)(t.bits >> (3 + 3 * g)) & 3u;
+        const uint32_t i = code == 1 ? n0 >> 1 : code == 2 ? n0 / 6u : n0;
+        *lo = i;
+        *hi = i + cnt - 1;
+        *res = code == 1 ? n0 & 1u : code == 2 ? n0 - 6u * i : 0u;
+        return;
+    }
+    const int q = g - kS1Seg;
+    const uint32_t A = (uint32_t)t.A, B = (uint32_t)t.B;
+    uint32_t j0 = 1, j1;
+    if ((t.bits & 3u) == EVAL_SINGLE) {
+        if (q >= 4) return;
+        j1 = q == 0 ? A / 6u : q == 1 ? A / 3u : q == 2 ? A / 2u : A;
+        if (q > 0) j0 = (q == 1 ? A / 6u : q == 2 ? A / 3u : A / 2u) + 1u;
+    } else {
+        const uint32_t Y = (q & 1) ? A : B, Z = (q & 1) ? B : A;  // this cut's and the previous one's
+        const int h = q >> 1, hp = (q - 1) >> 1;
+        j1 = h == 0 ? Y / 6u : h == 1 ? Y / 3u : h == 2 ? Y / 2u : Y;
+        if (q > 0) j0 = (hp == 0 ? Z / 6u : hp == 1 ? Z / 3u : hp == 2 ? Z / 2u : Z) + 1u;
+    }
+    if (j0 > j1) return;
+    *lo = j0 / 6u;
+    *hi = j1 / 6u;
+    *jr = make_uint2(j0, j1);
+}
+
+// Work units of segment g over the index range [ulo, uhi]; S2 blocks start on a multiple of
+// 32 positions (one Mobius word per warp load).
+__device__ __forceinline__ uint32_t tile_units(int g, uint32_t ulo, uint32_t uhi) {
+    if (ulo > uhi) return 0;
+    return g < kS1Seg ? (uhi - ulo) / kTileN + 1u : (uhi - (ulo & ~31u)) / kTileM + 1u;
 }
 
 // Constant part of an evaluation: 1 + kappa*M(A) (single) or

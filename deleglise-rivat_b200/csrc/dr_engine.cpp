@@ -840,8 +840,8 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
         sa.T.ckpt = (const int32_t*)c->bckpt.p;
         sa.T.cbase = cword0;
         CU(cudaMemsetAsync(c->ticket.p, 0, 8, c->stream));  // the work-queue counter (not the error flag)
-        launch_plan(sa.queries, sa.nq, sa.T, sa.n_slots, (u64*)c->ops.p, sa.acc, (i64*)c->counts.p, nullptr,
-                    (SlotDesc*)c->slots.p, c->sm_count, c->stream, S1Band{(u64)vlo + 1, (u64)vhi, 1});
+        launch_plan(sa.queries, sa.nq, sa.T, sa.n_blocks, (u64*)c->ops.p, sa.acc, (i64*)c->counts.p, nullptr,
+                    (SlotDesc*)c->slots.p, c->sm_count, c->stream, S1Band{(u64)vlo + 1, (u64)vhi, 1}, kPlanSlots);
         launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, sa.n_slots, (u64*)c->scan_tmp.p,
                         scan_u64_tmp_elems(sa.n_slots), c->stream);
         launch_sums(sa, grid, 256, c->stream);
@@ -856,7 +856,8 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
                     int* launches_out, const StreamPlan* sp = nullptr) {
     int rc;
     std::vector<QueryDev> qs((size_t)nq);
-    u64 slots = 0;
+    u64 slots = 0, blocks = 0;
+    bool rest = false;  // some evaluation may not fit the tile kernel
     int64_t inv_limit = 0;  // largest S1 divisor n worth tabulating
     for (int64_t i = 0; i < nq; ++i) {
         QueryDev& q = qs[(size_t)i];
@@ -866,8 +867,15 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         q.N = (X[i] <= c->t_u_total) ? 0 : X[i] / P[i].u_total;
         q.nc = num_candidates(q.N);
         q.slot_base = slots;
+        q.blk_base = blocks;
         slots += 2 * (u64)q.nc;
+        blocks += (u64)(q.nc + 31) / 32;
         if (q.N > 0) {
+            // Every evaluation has u <= y <= X.  Where cx^2 u >= 4 its S1 divisors stay below
+            // 1.4143 sqrt(X)/cx + 64, so with X < 2^51 and cx in this range every n and j is
+            // tabulated and below 2^31: the tile kernel takes them all (tile_eligible)
+            rest = rest || (u64)X[i] >= kTileMaxY || P[i].cx < 0.0625 || P[i].cx > 16.0 ||
+                   P[i].cx * P[i].cx * (double)P[i].u_total < 4.0;
             // S1 divisors stay below kappa_y ~ sqrt(y)/cx and the even correction's
             // 2*kappa_{y/2} ~ sqrt(2y)/cx; larger n (never expected) fall back to udiv
             const double b = 1.4143 * std::sqrt((double)X[i]) / P[i].cx + 64.0;
@@ -937,6 +945,8 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     }
     const TableView T = view_of(c);
     const int qn = (int)nq;
+    const S1Band band{0, sp ? (u64)sp->u_res : ~0ull, 0};
+    const bool tiles = !sw;  // the windowed S1 leaves every other lookup to the sums kernel
     CU(record_event(c, 2));
     CU(cudaMemcpyAsync(c->queries.p, sq, (size_t)nq * sizeof(QueryDev), cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemsetAsync(c->acc.p, 0, (size_t)nq * 3 * 8, c->stream));
@@ -950,9 +960,9 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         launch_inverse((double*)c->inv.p, inv_limit, (double2*)c->invw.p, invw_count, T.wheel, c->sm_count,
                        c->stream);
         // a streamed table: this pass takes the S1 lookups with q <= u_res, the bands the rest
-        launch_plan((const QueryDev*)c->queries.p, qn, T, slots, (u64*)c->ops.p, (u64*)c->acc.p, (i64*)c->counts.p,
-                    sw ? (S1WinDesc*)c->wdesc.p : nullptr, (SlotDesc*)c->slots.p, c->sm_count, c->stream,
-                    S1Band{0, sp ? (u64)sp->u_res : ~0ull, 0});
+        launch_plan((const QueryDev*)c->queries.p, qn, T, blocks, (u64*)c->ops.p, (u64*)c->acc.p, (i64*)c->counts.p,
+                    sw ? (S1WinDesc*)c->wdesc.p : nullptr, (SlotDesc*)c->slots.p, c->sm_count, c->stream, band,
+                    tiles ? kPlanTiles : kPlanSlots);
         launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
                         scan_u64_tmp_elems(slots), c->stream);
         launches += 5;
@@ -979,6 +989,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         sa.nq = qn;
         sa.T = T;
         sa.n_slots = slots;
+        sa.n_blocks = blocks;
         sa.prefix = (const u64*)c->prefix.p;
         sa.slots = (const SlotDesc*)c->slots.p;
         sa.ticket = (u64*)c->ticket.p;
@@ -991,9 +1002,24 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         int per_sm = 0;
         sums_kernel_occupancy(256, &per_sm);
         const int grid = c->sm_count * std::max(1, per_sm);
-        launch_sums(sa, grid, 256, c->stream);
+        if (tiles) {
+            launch_tiles(sa, c->sm_count, c->stream);
+            launches += 1;
+        }
+        if (tiles && rest) {
+            // what the tile kernel leaves (y >= 2^51: a few small k of an X above it)
+            launch_plan(sa.queries, qn, T, blocks, (u64*)c->ops.p, sa.acc, (i64*)c->counts.p, nullptr,
+                        (SlotDesc*)c->slots.p, c->sm_count, c->stream, band, kPlanRest);
+            launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
+                            scan_u64_tmp_elems(slots), c->stream);
+            CU(cudaMemsetAsync(c->ticket.p, 0, 8, c->stream));  // the work-queue counter (not the error flag)
+            launches += 4;
+        }
+        if (!tiles || rest) {
+            launch_sums(sa, grid, 256, c->stream);
+            launches += 1;
+        }
         CU(cudaGetLastError());
-        launches += 1;
         if (sp && sp->nbands > 0) {
             rc = stream_bands(c, *sp, sa, grid, &launches);
             if (rc) return rc;

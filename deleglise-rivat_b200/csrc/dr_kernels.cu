@@ -985,27 +985,44 @@ __device__ __forceinline__ u64 s1_compressed_lookups(const EvalDesc& d, const Ta
     return tot;
 }
 
-// counts[kCountsPerQuery*q + 0..4]: terms, evaluations, S1 lookups, S2 wheel
-// positions, compressed-tier S1 lookups -- summed over the warp before the atomics
-// (a band pass of a streamed table, band.s1_only, counts only its S1 lookups and adds
-// no constant part: those belong to the resident pass)
-__global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const TableView T, u64 n_slots,
+__device__ __forceinline__ int query_of_block(const QueryDev* q, int nq, u64 b) {
+    int lo = 0, hi = nq - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (q[mid].blk_base <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// One warp per (32-candidate block, evaluation e): lane l decodes candidate 32*block + l.
+// counts[kCountsPerQuery*q + 0..4]: terms, evaluations, S1 lookups, S2 wheel positions,
+// compressed-tier S1 lookups -- summed over the warp before the atomics (a band pass of a
+// streamed table, band.s1_only, counts only its S1 lookups and adds no constant part: those
+// belong to the resident pass).  mode:
+//   kPlanSlots  ops[s] = the slot's lookups and positions, for sums_kernel
+//   kPlanTiles  ops of a tile group's leader = its units, for the tile kernel; 0 elsewhere
+//   kPlanRest   ops[s] as kPlanSlots where the slot is not tile-eligible, else 0; the
+//               constants and counters were the kPlanTiles pass's
+__global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const TableView T, u64 n_blocks,
                             u64* __restrict__ ops, u64* __restrict__ acc, i64* __restrict__ counts,
-                            S1WinDesc* __restrict__ wdesc, SlotDesc* __restrict__ slots, const S1Band band) {
-    // whole warps step together (the stride is a multiple of 32), so the counters
-    // can be summed over the warp with every lane taking part
-    const u64 stride = (u64)gridDim.x * blockDim.x;
+                            S1WinDesc* __restrict__ wdesc, SlotDesc* __restrict__ slots, const S1Band band,
+                            const int mode) {
+    const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
     const int lane = threadIdx.x & 31;
-    for (u64 s0 = (u64)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); s0 < n_slots; s0 += stride) {
-        const u64 s = s0 + (u64)lane;
-        const bool valid = s < n_slots;
-        const int qi = query_of_slot(qs, nq, valid ? s : n_slots - 1);
+    for (u64 w = (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < 2 * n_blocks; w += warps) {
+        const int e = (int)(w & 1);
+        const int qi = query_of_block(qs, nq, w >> 1);
+        const QueryDev Q = qs[qi];
+        const u64 blk = (w >> 1) - Q.blk_base;
+        const i64 cand = (i64)(32 * blk) + lane;
+        const bool valid = cand < Q.nc;
+        const u64 s = Q.slot_base + 2 * (u64)cand + (u64)e;
         u64 v[7] = {0, 0, 0, 0, 0, 0, 0};  // C, terms, evaluations, S1, S2, compressed S1, S1 sum
+        u64 bits = 0;
         if (valid) {
-            const QueryDev Q = qs[qi];
-            const u64 local = s - Q.slot_base;
             EvalDesc d;
-            decode_eval(Q, T, (i64)(local >> 1), (int)(local & 1), d, band);
+            decode_eval(Q, T, cand, e, d, band);
             if (band.s1_only && d.kind != EVAL_NONE && d.total <= kBandInThread) {
                 // a band pass: nearly every evaluation has a handful of lookups in the band;
                 // this thread sums them (exact quotients, the band's view of the table), so
@@ -1021,27 +1038,28 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
                 for (int g = 0; g < kS1Seg; ++g) d.s1_cnt[g] = 0;
                 d.total = 0;
             }
-            ops[s] = d.total;
-            pack_slot(d, slots + s);
+            const bool tile = mode != kPlanSlots && tile_eligible(d, Q.inv_limit);
+            bits = pack_slot(d, slots + s, tile && mode == kPlanTiles ? kSlotTile : 0ull);
+            if (mode == kPlanSlots || mode == kPlanRest) ops[s] = tile ? 0ull : d.total;
             if (wdesc && Q.win) {
-                S1WinDesc w;
-                w.y = d.y;
+                S1WinDesc wd;
+                wd.y = d.y;
                 for (int g = 0; g < kS1Seg; ++g) {
                     const bool on = d.kind != EVAL_NONE && d.s1_full[g] > 0 && d.s1_wc[g] > 0;
-                    w.n0[g] = on ? (uint32_t)d.s1_n0[g] : 0u;
-                    w.cnt[g] = on ? (uint32_t)d.s1_full[g] : 0u;
-                    w.wc[g] = on ? (uint32_t)d.s1_wc[g] : 0u;
-                    w.w0[g] = on ? (uint32_t)(udiv(d.y, s1_n_at(d.s1_n0[g], d.s1_stride[g], (u64)(d.s1_full[g] - 1))) /
-                                              Q.win)
-                                 : 0u;
-                    w.sg[g] = on ? (int32_t)(d.coef * d.s1_sign[g]) * d.s1_stride[g] : 0;
+                    wd.n0[g] = on ? (uint32_t)d.s1_n0[g] : 0u;
+                    wd.cnt[g] = on ? (uint32_t)d.s1_full[g] : 0u;
+                    wd.wc[g] = on ? (uint32_t)d.s1_wc[g] : 0u;
+                    wd.w0[g] = on ? (uint32_t)(udiv(d.y, s1_n_at(d.s1_n0[g], d.s1_stride[g], (u64)(d.s1_full[g] - 1))) /
+                                               Q.win)
+                                  : 0u;
+                    wd.sg[g] = on ? (int32_t)(d.coef * d.s1_sign[g]) * d.s1_stride[g] : 0;
                 }
-                wdesc[s] = w;
+                wdesc[s] = wd;
             }
             if (d.kind != EVAL_NONE) {
                 if (!band.s1_only) {
                     v[0] = (u64)(d.coef * eval_constant(d, T));
-                    v[1] = (local & 1) == 0 ? 1 : 0;
+                    v[1] = e == 0 ? 1 : 0;
                     v[2] = 1;
                 }
                 u64 s1d = 0, s1f = 0;  // lookups left to the sums kernel, all lookups
@@ -1054,19 +1072,35 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
                 v[5] = s1_compressed_lookups(d, T);
             }
         }
-        // one atomic per counter and warp where all its slots belong to one query
-        const int q0 = __shfl_sync(0xffffffffu, qi, 0);
-        if (__all_sync(0xffffffffu, qi == q0)) {
+        if (mode == kPlanTiles) {
+            // the block's groups: one, or a few where the block straddles a range boundary
+            u64 units = 0;
+            SlotDesc t = {};
+            if (bits & kSlotTile) t = slots[s];
+            unsigned left = __ballot_sync(0xffffffffu, (bits & kSlotTile) != 0);
+            while (left) {
+                const int lead = __ffs(left) - 1;
+                const u64 sig = __shfl_sync(0xffffffffu, bits & (kSlotTile | kTileSig), lead);
+                const bool member = (bits & (kSlotTile | kTileSig)) == sig;
+                left &= ~__ballot_sync(0xffffffffu, member);
+                uint32_t sum = 0;
 #pragma unroll
-            for (int i = 0; i < 7; ++i) v[i] = warp_sum_u64(v[i]);
-            if (lane == 0) {
-                atomicAdd(acc + 3 * qi, v[0]);
-                if (v[6]) atomicAdd(acc + 3 * qi + 1, v[6]);
-                unsigned long long* cq = reinterpret_cast<unsigned long long*>(counts + kCountsPerQuery * qi);
-                for (int i = 0; i < 5; ++i)
-                    if (v[i + 1]) atomicAdd(cq + i, v[i + 1]);
+                for (int g = 0; g < kS1Seg + 8; ++g) {
+                    uint32_t lo = 1, hi = 0, res;
+                    uint2 jr;
+                    if (member) tile_range(t, g, &lo, &hi, &res, &jr);
+                    const uint32_t ulo = __reduce_min_sync(0xffffffffu, lo <= hi ? lo : 0xffffffffu);
+                    const uint32_t uhi = __reduce_max_sync(0xffffffffu, lo <= hi ? hi : 0u);
+                    sum += tile_units(g, ulo, uhi);
+                }
+                if (lane == lead) units = sum;
             }
-        } else if (valid) {
+            if (valid) ops[s] = units;
+        }
+        if (mode == kPlanRest) continue;
+#pragma unroll
+        for (int i = 0; i < 7; ++i) v[i] = warp_sum_u64(v[i]);
+        if (lane == 0) {
             if (v[0]) atomicAdd(acc + 3 * qi, v[0]);
             if (v[6]) atomicAdd(acc + 3 * qi + 1, v[6]);
             unsigned long long* cq = reinterpret_cast<unsigned long long*>(counts + kCountsPerQuery * qi);
@@ -1076,11 +1110,11 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
     }
 }
 
-void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_slots, u64* ops, u64* acc, i64* counts,
-                 S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s, const S1Band& band) {
-    if (n_slots == 0) return;
-    const int grid = (int)std::min<u64>((n_slots + 127) / 128, (u64)sm_count * 16);
-    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_slots, ops, acc, counts, wdesc, slots, band);
+void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc, i64* counts,
+                 S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s, const S1Band& band, int mode) {
+    if (n_blocks == 0) return;
+    const int grid = (int)std::min<u64>((2 * n_blocks + 3) / 4, (u64)sm_count * 16);
+    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode);
 }
 
 // Direct answers for queries with X <= table u_total (get_M, :1465-1467).

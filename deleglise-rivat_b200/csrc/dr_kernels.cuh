@@ -96,6 +96,7 @@ struct SumsArgs {
     int nq;
     TableView T;
     u64 n_slots;
+    u64 n_blocks;       // 32-candidate blocks of all queries
     const u64* prefix;  // [n_slots + 1] exclusive op prefix
     const SlotDesc* slots;  // [n_slots] each slot's evaluation, written by plan_kernel
     u64* ticket;        // [0]: work-queue counter, [1]: error flag; zeroed before launch
@@ -159,14 +160,19 @@ constexpr int kCountsPerQuery = 5;
 // A band pass of a streamed table: evaluations with at most this many S1 lookups in the
 // band are summed by the planning thread itself (ops 0 for the sums kernel).
 constexpr int kBandInThread = 64;
-void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_slots, u64* ops, u64* acc,
+// What a planning pass leaves in ops (plan_kernel): work for the sums kernel (every slot),
+// for the tile kernel, or for the sums kernel where the tile kernel takes nothing.
+enum { kPlanSlots = 0, kPlanTiles = 1, kPlanRest = 2 };
+void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc,
                  i64* counts, S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s,
-                 const S1Band& band = S1Band{0, ~0ull, 0});
+                 const S1Band& band, int mode);
 // Windowed S1 (window length win: a power of two, 2^12 .. 2^16).
 void launch_s1win(const S1WinArgs& a, u64 win, int sm_count, cudaStream_t s);
 void launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t tmp_elems, cudaStream_t s);
 size_t scan_u64_tmp_elems(u64 n);
 void launch_sums(const SumsArgs& a, int grid, int block, cudaStream_t s);
+// The tile kernel (dr_tiles.cu) on the ops of a kPlanTiles pass.
+void launch_tiles(const SumsArgs& a, int sm_count, cudaStream_t s);
 // Reciprocal tables shared by every evaluation of a launch.
 void launch_inverse(double* rcp, i64 inv_limit, double2* invw, i64 invw_count, const uint4* wheel, int sm_count,
                     cudaStream_t s);
