@@ -44,6 +44,10 @@ int fail(int code, const char* fmt, ...) {
                         __FILE__, __LINE__);                                                  \
     } while (0)
 
+// Sieving primes up to which squares are not bucketed: the buckets' five launches take about
+// 20 us, the squares in the sieve itself less up to about 1.5e9 values (1e6 values 0.046 ->
+// 0.024 ms, 1e9 0.948 -> 0.919 ms; 2e9 the same, 5.4e9 4.42 -> 4.50 ms).
+constexpr size_t kBucketMinPrimes = 4096;
 constexpr int64_t kDenseInt16Limit = 7600000000LL;  // |M(n)| < 32768 for n <= 7.6e9
 
 struct DevBuf {
@@ -273,10 +277,23 @@ int64_t split_point_host(double cx, int64_t y) {
     return A;
 }
 
-int pick_segment(const dr_params* p) {
-    int lg = (p && p->segment_log2) ? p->segment_log2 : 18;
+// Sieve shape: values per segment and threads per CTA.  Where the caller leaves both open, a
+// table below 1.5e8 values takes 256-thread CTAs on about 700 segments, so that it spreads
+// over the whole GPU (measured, all-dense table: 1e6 values 0.119 ms with 2^18 x 1024, one
+// segment per CTA and 4 CTAs in all -> 0.046 ms with 2^12 x 256; 1e7: 0.138 -> 0.068 ms with
+// 2^14 x 256; 1e8: 0.273 -> 0.272 ms with 2^16 x 256); from there on the large segments win
+// (3e8: 0.593 ms with 2^18 x 1024, 0.597 ms with 2^16 x 256).
+void pick_shape(int64_t u_total, const dr_params* p, int* S, int* block) {
+    int lg = p ? p->segment_log2 : 0, b = p ? p->block_threads : 0;
+    if (lg == 0 && b == 0 && u_total < 150000000) {
+        lg = 12;
+        while (lg < 16 && (700ll << lg) * 1.4 < (double)u_total) ++lg;
+        b = 256;
+    }
+    if (lg == 0) lg = 18;
     lg = std::max(12, std::min(lg, 18));
-    return 1 << lg;
+    *S = 1 << lg;
+    *block = b ? b : 1024;
 }
 
 TableView view_of(dr_ctx* c) {
@@ -336,8 +353,8 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     // freed and regrown, or a launch fail partway): the table is valid again only
     // once every launch of this build has been enqueued.
     c->table_valid = false;
-    const int S = pick_segment(tuning);
-    const int block = (tuning && tuning->block_threads) ? tuning->block_threads : 1024;
+    int S, block;
+    pick_shape(u_total, tuning, &S, &block);
     if (block < 128 || block > 1024 || (block & 31))
         return fail(DR_ERR_PARAMS, "block_threads must be a multiple of 32 in [128, 1024]");
     const int64_t comp = u_total - u_dense;
@@ -401,6 +418,9 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     a.sq_off = nullptr;
     a.sq_seg0 = 0;
     a.sq_pos = nullptr;
+    // few primes: their squares are marked by the sieve, a prime per thread
+    if (pr.size() <= kBucketMinPrimes) sq_hits = 0;
+    if (sq_hits == 0) a.sqC_first = (int)pr.size();
     if (sq_hits > 0) {
         if ((rc = ensure(c, c->sq_cnt, (size_t)nseg * 8))) return rc;
         if ((rc = ensure(c, c->sq_cur, (size_t)nseg * 8))) return rc;
@@ -472,6 +492,14 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
         launch_sieve(m, l.odd, (int)std::max<int64_t>(1, std::min<int64_t>(l.end - l.begin, l.odd ? grid_o : grid_f)),
                      block, l.odd ? smem_o : smem_f, c->stream);
         CU(cudaGetLastError());
+        if (plan.size() == 1) {  // nothing to overlap: no side stream
+            launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, 0, l.end, 1024, c->stream);
+            launch_fixup_range((int16_t*)c->dM.p, u_dense, S, (const int32_t*)c->seg_off.p, (int32_t*)c->ckpt.p,
+                               nwords, dense_segs, 0, l.end, c->sm_count * 16, c->stream);
+            CU(cudaGetLastError());
+            launches += 2;
+            break;
+        }
         if (forks < dr_ctx::kForks - 1 || li + 1 == plan.size()) {
             CU(cudaEventRecord(c->fork[forks], c->stream));
             CU(cudaStreamWaitEvent(c->side, c->fork[forks], 0));
@@ -489,8 +517,10 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
             launches += 2;
         }
     }
-    CU(cudaEventRecord(c->join, c->side));
-    CU(cudaStreamWaitEvent(c->stream, c->join, 0));
+    if (plan.size() > 1) {
+        CU(cudaEventRecord(c->join, c->side));
+        CU(cudaStreamWaitEvent(c->stream, c->join, 0));
+    }
     launches += (int)plan.size() - 3;
     CU(record_event(c, 1));
 
@@ -676,7 +706,9 @@ bool band_odd(const StreamPlan& sp, int64_t vlo, int64_t vhi) {
 // resident build (nothing may grow once launches are queued: the segment offsets of the
 // resident table carry into the first band).  *sp.nbands == 0: no streaming.
 int plan_stream(dr_ctx* c, int64_t X, int64_t ut, int64_t ud, int64_t ml, const dr_params& tune, StreamPlan* sp) {
-    stream_geometry(ut, ud, pick_segment(&tune), c->u_resident, c->band_values, sp);
+    int S0, block;
+    pick_shape(ut, &tune, &S0, &block);
+    stream_geometry(ut, ud, S0, c->u_resident, c->band_values, sp);
     if (sp->nbands == 0) return DR_OK;
     if (X <= ut) {
         *sp = StreamPlan{};
@@ -684,7 +716,7 @@ int plan_stream(dr_ctx* c, int64_t X, int64_t ut, int64_t ud, int64_t ml, const 
                     (long long)ut);
     }
     const int64_t S = sp->S;
-    sp->block = tune.block_threads ? tune.block_threads : 1024;
+    sp->block = block;
     sp->mu_limit = ml;
     if (ml > sp->u_res) {
         *sp = StreamPlan{};
@@ -1435,7 +1467,12 @@ int dr_mertens_batch(dr_ctx* c, const int64_t* X, int64_t count, const dr_params
         const bool streamed = sp.nbands > 0;
         const size_t n_res = streamed ? primes_upto(c, isqrt_i64(sp.u_res)).size() : 0;
         if (!rc) rc = stage_reserve(c, stage_bytes_for(n_primes + n_res, count) + (streamed ? kMaxSieveItems * 16 : 0));
-        if (!rc) rc = build_table(c, streamed ? sp.u_res : ut, ud, ml, &tune, st);
+        dr_params shape = tune;
+        if (streamed) {  // the resident part has the whole table's segments
+            shape.segment_log2 = 63 - __builtin_clzll((unsigned long long)sp.S);
+            shape.block_threads = sp.block;
+        }
+        if (!rc) rc = build_table(c, streamed ? sp.u_res : ut, ud, ml, &shape, st);
         if (!rc) rc = enqueue_queries(c, X, P.data(), count, &tune, &launches, streamed ? &sp : nullptr);
         if (!rc) break;
     }

@@ -716,11 +716,14 @@ int sieve_items_prefix(const uint4* items, int n_items, int n_primes) {
 
 void sieve_kernel_attrs(size_t smem, bool odd, int block, int* per_sm) {
     *per_sm = 0;
+    // the opt-in limit is the kernel's, for every context and shape: always the largest
     if (odd) {
-        cudaFuncSetAttribute(sieve_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(sieve_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sieve_smem_bytes(1 << 18, true));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sieve_kernel<true>, block, smem);
     } else {
-        cudaFuncSetAttribute(sieve_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(sieve_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sieve_smem_bytes(1 << 18, false));
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sieve_kernel<false>, block, smem);
     }
 }

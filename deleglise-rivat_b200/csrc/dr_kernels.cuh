@@ -183,8 +183,8 @@ void launch_table_sums(const TableView& T, i64 nwords, u64* out6, int sm_count, 
 void init_piece_constants();
 // Record a message for dr_last_error() (fixed thread-local buffer) and return code.
 int record_error(int code, const char* msg);
-// Opt the sieve kernel into `smem` bytes of dynamic shared memory and report
-// how many CTAs of `block` threads fit on one SM.
+// Opt the sieve kernel into the shared memory of every segment length and report how many
+// CTAs of `block` threads with `smem` bytes fit on one SM.
 void sieve_kernel_attrs(size_t smem, bool odd, int block, int* per_sm);
 // Segments [a, b) of an odd-mode launch that may follow launches covering [0, a):
 // the largest b such that the halves of every value of [a, b) lie below segment a.
