@@ -171,7 +171,7 @@ int dr_mlp_get_weights(dr_mlp *mlp, float *w, int64_t count);
 int dr_mlp_forward(dr_mlp *mlp, const float *x, int64_t B, float *y);
 /* Gradient of the mean squared error over B examples (no update). */
 int dr_mlp_grad(dr_mlp *mlp, const float *x, const float *t, int64_t B, float *grad, float *loss);
-/* `steps` full-batch Adam updates (each one replay of a captured CUDA graph). */
+/* `steps` full-batch Adam updates (one kernel launch). */
 int dr_mlp_train(dr_mlp *mlp, const float *x, const float *t, int64_t B, int steps, float lr,
                  float *final_loss);
 int dr_tuner_features(int64_t X, uint64_t hbm_budget, int sm_count, int batch, float *out4);
