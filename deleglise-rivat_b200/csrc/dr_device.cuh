@@ -6,6 +6,7 @@
 // mertens_dr.hpp:<line> (ecreeth/deleglise-rivat).
 #pragma once
 
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -208,6 +209,7 @@ struct QueryDev {
     u64 win;        // S1 window length W (a power of two; 0: no windowed S1)
     u64 win_max;    // windows w < win_max lie in the dense tier ((w+1)*W <= u_dense < 2^31)
     u64 inv_limit;  // largest tabulated S1 reciprocal 1/n
+    u64 twin_max;   // windows of kTileWin table values the window kernel may use (0: none)
 };
 
 #ifndef DRB_WIN_MIN
@@ -323,8 +325,30 @@ constexpr u64 kSlotS1Only = 1ull << 15;
 constexpr u64 kSlotTile = 1ull << 16;
 constexpr uint32_t kTileN = 128;
 constexpr uint32_t kTileM = 64;
+constexpr uint32_t kTileS1Units = 8;
 // y below this: one FMA rounded down gives every quotient of the tile kernel exactly
 constexpr u64 kTileMaxY = 1ull << 51;
+
+// The S1 lookups M(q) of a block with q below tile_windows() * kTileWin are the window
+// kernel's.  Windows stop where one of them holds fewer than kWinRun odd divisors of the
+// block's first candidate (y W / (2 q^2) = kWinRun), and at the query's last window.  IEEE
+// operations only: host and device agree.
+constexpr int kTileWin = 98304;
+constexpr double kWinRun = 64.0;
+__host__ __device__ inline u64 tile_windows(u64 X, u64 blk, u64 twin_max) {
+    const double y = (double)X / (double)(96 * blk + 1);
+    const double w = sqrt(y * (1.0 / (2.0 * kWinRun * kTileWin)));
+    return w < (double)twin_max ? (u64)w : twin_max;
+}
+
+// A tile group as the window kernel (dr_windows.cu) reads it.
+struct __align__(16) WinGroup {
+    uint32_t ulo[kS1Seg], uhi[kS1Seg];  // union of the members' index ranges (tile_range's units)
+    uint32_t mm;    // lanes (candidates of the block) that are members
+    uint32_t wc;    // windows w < wc
+    uint32_t bits;  // stride codes, as SlotDesc.bits
+    uint32_t pad;
+};
 
 #ifdef __CUDACC__
 __device__ __forceinline__ i64 piece_mcount(i64 lo, i64 hi) {
@@ -540,7 +564,8 @@ __device__ __forceinline__ int stride_of_code(u64 c) { return c == 0 ? 1 : c == 
 
 // An evaluation as the sums kernels need it, written once by the planner, with `flags` set
 // in its bits; returns the bits.
-__device__ __forceinline__ u64 pack_slot(const EvalDesc& d, SlotDesc* out, u64 flags) {
+// (near: lookups of each S1 segment left to the window kernel, kept in the high word of cnt)
+__device__ __forceinline__ u64 pack_slot(const EvalDesc& d, SlotDesc* out, u64 flags, const uint32_t* near = nullptr) {
     SlotDesc s;
     if (d.kind == EVAL_NONE) {  // no terms
         s.y = 0;
@@ -556,7 +581,7 @@ __device__ __forceinline__ u64 pack_slot(const EvalDesc& d, SlotDesc* out, u64 f
     u64 bits = (u64)d.kind | (d.coef < 0 ? 4ull : 0ull) | (d.npieces == 0 ? kSlotS1Only : 0ull) | flags;
     for (int g = 0; g < kS1Seg; ++g) {
         s.n0[g] = d.s1_n0[g];
-        s.cnt[g] = d.s1_cnt[g];
+        s.cnt[g] = near ? d.s1_cnt[g] | (i64)((u64)near[g] << 32) : d.s1_cnt[g];
         bits |= (stride_code(d.s1_stride[g]) | (d.s1_sign[g] < 0 ? 4ull : 0ull)) << (3 + 3 * g);
     }
     s.bits = bits;
@@ -606,6 +631,27 @@ __device__ __forceinline__ bool tile_eligible(const EvalDesc& d, u64 inv_limit) 
 // the stride codes (then their S1 segments lie on the same arithmetic progressions).
 constexpr u64 kTileSig = 3ull | (3ull << 3) | (3ull << 6) | (3ull << 9) | (3ull << 12);
 
+// Index range of S1 segment g of a tile slot, the window kernel's lookups included.
+__device__ __forceinline__ void win_range(const SlotDesc& t, int g, uint32_t* lo, uint32_t* hi, uint32_t* res) {
+    const uint32_t cnt = (uint32_t)t.cnt[g] + (uint32_t)((u64)t.cnt[g] >> 32), n0 = (uint32_t)t.n0[g];
+    const uint32_t code = (uint32_t)(t.bits >> (3 + 3 * g)) & 3u;
+    const uint32_t i = code == 1 ? n0 >> 1 : code == 2 ? n0 / 6u : n0;
+    *lo = i;
+    *hi = i + cnt - 1;
+    *res = code == 1 ? n0 & 1u : code == 2 ? n0 - 6u * i : 0u;
+    if (cnt == 0) *lo = 1, *hi = 0;
+}
+
+// divisor of index i in an S1 segment of stride code `code` (1, 2, 6, wheel)
+__device__ __forceinline__ uint32_t tile_n(uint32_t code, uint32_t i, uint32_t res) {
+    return code == 0 ? i : code == 1 ? 2u * i + res : code == 2 ? 6u * i + res : 3u * i + 1u + (i & 1u);
+}
+
+// floor(y/n) in the low word: yd = y + 1/2 < 2^51, r = RN(1/n) (dr_tiles.cu)
+__device__ __forceinline__ uint32_t floor_q(double yd, double r) {
+    return (uint32_t)__double2loint(__fma_rd(yd, r, 4503599627370496.0));
+}
+
 // Range [lo, hi] of segment g of a tile slot (lo > hi: empty), in the units the tile kernel
 // counts: S1 segments (g < kS1Seg) by i with n = stride*i + *res (the wheel: n =
 // candidate_k(i)), S2 pieces by wheel position, with the piece's j range in jr.
@@ -646,10 +692,11 @@ __device__ __forceinline__ void tile_range(const SlotDesc& t, int g, uint32_t* l
 }
 
 // Work units of segment g over the index range [ulo, uhi]; S2 blocks start on a multiple of
-// 32 positions (one Mobius word per warp load).
+// 32 positions (one Mobius word per warp load).  An S1 block counts kTileS1Units: its gathers
+// take that much longer than an S2 block.
 __device__ __forceinline__ uint32_t tile_units(int g, uint32_t ulo, uint32_t uhi) {
     if (ulo > uhi) return 0;
-    return g < kS1Seg ? (uhi - ulo) / kTileN + 1u : (uhi - (ulo & ~31u)) / kTileM + 1u;
+    return g < kS1Seg ? kTileS1Units * ((uhi - ulo) / kTileN + 1u) : (uhi - (ulo & ~31u)) / kTileM + 1u;
 }
 
 // Constant part of an evaluation: 1 + kappa*M(A) (single) or

@@ -48,6 +48,11 @@ int fail(int code, const char* fmt, ...) {
 // 20 us, the squares in the sieve itself less up to about 1.5e9 values (1e6 values 0.046 ->
 // 0.024 ms, 1e9 0.948 -> 0.919 ms; 2e9 the same, 5.4e9 4.42 -> 4.50 ms).
 constexpr size_t kBucketMinPrimes = 4096;
+// The window kernel takes S1 lookups where a launch has this many of them, from queries of at
+// least kWinMinX (sums phase without -> with it: X = 10^14 1.37 -> 1.58 ms, 10^14.5 2.83 -> 2.59
+// ms at about 2.4e9 lookups, 10^15 5.3 -> 4.8, 10^16 25.9 -> 21.6, 10^17 136 -> 101 ms).
+constexpr double kWinMinLookups = 2e9;
+constexpr int64_t kWinMinX = 1000000000000LL;
 constexpr int64_t kDenseInt16Limit = 7600000000LL;  // |M(n)| < 32768 for n <= 7.6e9
 
 struct DevBuf {
@@ -83,6 +88,7 @@ struct dr_ctx {
     int64_t last_bands = 0;        // bands the enqueued call streams
     // query buffers
     DevBuf queries, ops, prefix, scan_tmp, acc, counts, ticket, misc, inv, invw, wdesc, witems, slots;
+    DevBuf groups, titems;  // window kernel: tile groups; work items and tasks
     // table state
     bool table_valid = false;
     int64_t t_u_total = 0, t_u_dense = 0, t_mu_limit = 0, t_nwords = 0;
@@ -110,6 +116,9 @@ struct dr_ctx {
     // pinned copy of the windowed-S1 work items (single queries only, never captured)
     S1WinItem* wstage = nullptr;
     size_t wstage_cap = 0, wstage_used = 0;
+    // pinned copy of the window kernel's items and tasks (a graph owns its own)
+    uint8_t* tstage = nullptr;
+    size_t tstage_cap = 0, tstage_used = 0;
     bool capturing = false;
     struct Graph {
         std::vector<int64_t> X;
@@ -117,6 +126,7 @@ struct dr_ctx {
         dr_params tune;
         cudaGraphExec_t exec = nullptr;
         uint8_t* stage = nullptr;
+        uint8_t* tstage = nullptr;
         int launches = 0;
     };
     std::vector<Graph> graphs;  // replayable batch pipelines, most recent last
@@ -129,6 +139,7 @@ void drop_graphs(dr_ctx* c) {
     for (auto& g : c->graphs) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         if (g.stage) cudaFreeHost(g.stage);
+        if (g.tstage) cudaFreeHost(g.tstage);
     }
     c->graphs.clear();
 }
@@ -182,7 +193,7 @@ bool release_scratch(dr_ctx* c) {
                       &c->items, &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->counts, &c->ticket,
                       &c->misc, &c->inv, &c->invw, &c->wdesc, &c->witems, &c->slots, &c->prcp, &c->sq_cnt,
                       &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp, &c->items_odd, &c->dplanes, &c->bplanes,
-                      &c->bckpt};
+                      &c->bckpt, &c->groups, &c->titems};
     bool any = false;
     for (DevBuf* b : bufs) {
         any = any || b->p;
@@ -884,6 +895,119 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
     return DR_OK;
 }
 
+// Windows of kTileWin table values the window kernel may use for a query: inside the dense
+// tier and below 2^31; none where the query is too small to gain from them.  A window at q
+// holds about X W / (2 q^2) lookups in all; one with fewer than 2^18 is not worth its staging.
+u64 window_limit(int64_t X, const dr_params& p, int64_t u_dense) {
+    if (X <= p.u_total || p.u_total < 1 || X < kWinMinX) return 0;
+    const double q = std::sqrt((double)X * (double)kTileWin / (2.0 * 262144.0));
+    return (u64)(std::min(q, (double)std::min<int64_t>(u_dense, (int64_t(1) << 31) - 1)) / (double)kTileWin);
+}
+
+struct WindowWork {
+    std::vector<TileWinItem> items;
+    std::vector<uint32_t> w;  // window of each item
+    std::vector<float> cost;  // its lookups, about
+    std::vector<TileWinTask> tasks;
+};
+
+// Items of the window kernel for one query: for each window the blocks whose windows include
+// it (tile_windows), less the leading ones whose quotients all lie above it, in runs of at
+// most `task` lookups by an estimate of each block's lookups in the window -- 29 members, the
+// divisors n = y/q of the window at every second or so, y = X/k and (for k <= N/3) y/3,
+// quotients from about cx sqrt(y/2) on.  A group of more than kWinUnit lookups falls into
+// pieces, so that a warp's unit stays short against a task.
+void window_items(const QueryDev& q, int qi, double task, WindowWork& out) {
+    const u64 nb = (u64)(q.nc + 31) / 32;
+    if (q.twin_max == 0 || nb == 0) return;
+    constexpr double kWinUnit = 65536.0;
+    const double X = (double)q.X, W = (double)kTileWin;
+    for (u64 w = 0;; ++w) {
+        if (tile_windows(q.X, 0, q.twin_max) <= w) break;
+        u64 lo = 1, hi = nb;  // blocks with tile_windows > w: [0, hi) (it falls with the block)
+        while (lo < hi) {
+            const u64 mid = (lo + hi + 1) / 2;
+            if (tile_windows(q.X, mid - 1, q.twin_max) > w) lo = mid;
+            else hi = mid - 1;
+        }
+        const double q0 = W * (double)w, q1 = q0 + W;
+        // smallest quotient of y: its largest divisor is at most 1.4143 sqrt(y)/cx + 64
+        const double qs = q1 / (0.65 * q.cx);
+        const double kmin = X / (3.0 * qs * qs + 1e4 * q1);
+        u64 b = kmin > 192.0 ? (u64)(kmin / 96.0) - 1 : 0;
+        while (b < lo) {
+            auto cost = [&](double k, double third) {
+                const double y = X / (k * third), qa = std::max(q0, 0.7 * q.cx * std::sqrt(y));
+                // single evaluations (k > N/2) take every n
+                const double den = third == 1.0 && k * 2.0 > (double)q.N ? 29.0 : 12.0;
+                return k * third > (double)q.N || qa >= q1 ? 0.0 : den * y * (1.0 / qa - 1.0 / q1);
+            };
+            double t = 4000.0;
+            const int points = b < 4 ? 8 : 1;  // a leading block's k vary too much for its middle
+            for (int j = 0; j < points; ++j) {
+                const double k = 96.0 * ((double)b + (j + 0.5) / points);
+                t += (cost(k, 1.0) + cost(k, 3.0)) * (b == 0 ? 2.0 : 1.0) / points;
+            }
+            u64 n = std::max<u64>(1, (u64)(task / t));
+            n = std::min(std::min(n, b / 2 + 1), lo - b);  // the estimate holds near b
+            TileWinItem it{(uint32_t)(q.blk_base + b), (uint32_t)(q.blk_base + b + n), (uint32_t)qi,
+                           (uint32_t)std::min(1.0 + t / (2.0 * kWinUnit), 1024.0), 0};
+            out.items.push_back(it);
+            out.w.push_back((uint32_t)w);
+            out.cost.push_back((float)(t * (double)n));
+            b += n;
+        }
+    }
+}
+
+// The window kernel's work for a launch: items of every query, in order of their windows (one
+// staging serves all queries), and tasks of consecutive items of one window.
+void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P, int64_t u_dense, int sm_count,
+                 WindowWork& out) {
+    double total = 0.0;
+    for (size_t i = 0; i < qs.size(); ++i)
+        if (qs[i].N > 0 && X[i] >= kWinMinX)
+            total += 0.53 * std::sqrt((double)X[i] * (double)qs[i].N) / P[i].cx;  // S1 lookups, about
+    if (total < kWinMinLookups) return;
+    const double task = std::max(total / (sm_count * 12.0), 524288.0);  // a dozen to a CTA
+    for (size_t i = 0; i < qs.size(); ++i)
+        if ((qs[i].twin_max = window_limit(X[i], P[i], u_dense))) window_items(qs[i], (int)i, task, out);
+    const size_t n = out.items.size();
+    if (qs.size() > 1) {
+        std::vector<uint32_t> at(n);
+        for (size_t i = 0; i < n; ++i) at[i] = (uint32_t)i;
+        std::stable_sort(at.begin(), at.end(), [&](uint32_t a, uint32_t b) { return out.w[a] < out.w[b]; });
+        WindowWork s;
+        for (uint32_t i : at) {
+            s.items.push_back(out.items[i]);
+            s.w.push_back(out.w[i]);
+            s.cost.push_back(out.cost[i]);
+        }
+        out = std::move(s);
+    }
+    std::vector<float> tcost;
+    for (size_t i = 0; i < n;) {
+        size_t j = i;
+        double t = 0.0;
+        uint32_t u = 0;
+        while (j < n && out.w[j] == out.w[i] && t < task) {
+            out.items[j].u0 = u;
+            u += 2 * (out.items[j].b1 - out.items[j].b0) * out.items[j].parts;
+            t += out.cost[j++];
+        }
+        out.tasks.push_back(TileWinTask{out.w[i], (uint32_t)i, (uint32_t)j, u});
+        tcost.push_back((float)t);
+        i = j;
+    }
+    // the longest first, so that the last ones are short
+    std::vector<uint32_t> at(out.tasks.size());
+    for (size_t i = 0; i < at.size(); ++i) at[i] = (uint32_t)i;
+    std::stable_sort(at.begin(), at.end(), [&](uint32_t a, uint32_t b) { return tcost[a] > tcost[b]; });
+    std::vector<TileWinTask> sorted;
+    for (uint32_t i : at) sorted.push_back(out.tasks[i]);
+    out.tasks = std::move(sorted);
+}
+
 int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, const dr_params* tuning,
                     int* launches_out, const StreamPlan* sp = nullptr) {
     int rc;
@@ -919,6 +1043,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     for (int64_t i = 0; i < nq; ++i) {
         QueryDev& q = qs[(size_t)i];
         q.inv_limit = (u64)inv_limit;
+        q.twin_max = 0;
         q.win = q.win_max = 0;
         // opt-in: since the S1 terms that cancel between a candidate's two evaluations
         // are left out, the direct S1 is faster at every X measured (10^15 .. 10^18)
@@ -931,6 +1056,19 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         q.win = (u64)W;
         witems = s1win_items(q, (int)i);
         if (witems.empty()) q.win = q.win_max = 0;
+    }
+    // the window kernel's work
+    WindowWork ww;
+    if (witems.empty() && blocks > 0) {
+        window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
+        // buffers beyond what the call needs anyway: without room for them the tile kernel
+        // takes these lookups too
+        if (!ww.tasks.empty() && (ensure(c, c->groups, (size_t)blocks * 2 * sizeof(WinGroup)) ||
+                                  ensure(c, c->titems, ww.items.size() * sizeof(TileWinItem) + 16 +
+                                                           ww.tasks.size() * sizeof(TileWinTask)))) {
+            for (QueryDev& q : qs) q.twin_max = 0;
+            ww.tasks.clear();
+        }
     }
     const int64_t invw_count = c->t_mu_limit / 6 + 1;  // every S2 j <= A <= mu_limit
     if ((rc = ensure(c, c->queries, (size_t)nq * sizeof(QueryDev)))) return rc;
@@ -958,6 +1096,22 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     }
     const void* sq = stage_put(c, qs.data(), (size_t)nq * sizeof(QueryDev));
     if (!sq) return fail(DR_ERR_NOMEM, "internal: staging area too small");
+    const size_t item_bytes = (ww.items.size() * sizeof(TileWinItem) + 15) & ~size_t(15);
+    const bool windows = !ww.tasks.empty();
+    c->tstage_used = windows ? item_bytes + ww.tasks.size() * sizeof(TileWinTask) : 0;
+    if (windows) {
+        if (c->tstage_cap < c->tstage_used) {  // the previous call's copies have completed (it synchronised)
+            if (c->capturing) return fail(DR_ERR_ARG, "internal: staging growth during graph capture");
+            if (c->tstage) cudaFreeHost(c->tstage);
+            c->tstage = nullptr;
+            c->tstage_cap = 0;
+            const size_t cap = c->tstage_used + c->tstage_used / 4;
+            CU(cudaMallocHost((void**)&c->tstage, cap));
+            c->tstage_cap = cap;
+        }
+        std::memcpy(c->tstage, ww.items.data(), ww.items.size() * sizeof(TileWinItem));
+        std::memcpy(c->tstage + item_bytes, ww.tasks.data(), ww.tasks.size() * sizeof(TileWinTask));
+    }
     const void* sw = nullptr;
     c->wstage_used = 0;
     c->last_bands = 0;
@@ -986,6 +1140,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     CU(cudaMemsetAsync(c->ticket.p, 0, 32, c->stream));
     if (sw)
         CU(cudaMemcpyAsync(c->witems.p, sw, witems.size() * sizeof(S1WinItem), cudaMemcpyHostToDevice, c->stream));
+    if (windows) CU(cudaMemcpyAsync(c->titems.p, c->tstage, c->tstage_used, cudaMemcpyHostToDevice, c->stream));
     launch_direct((const QueryDev*)c->queries.p, qn, T, (u64*)c->acc.p, c->stream);
     int launches = 1;
     if (slots > 0) {
@@ -994,7 +1149,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         // a streamed table: this pass takes the S1 lookups with q <= u_res, the bands the rest
         launch_plan((const QueryDev*)c->queries.p, qn, T, blocks, (u64*)c->ops.p, (u64*)c->acc.p, (i64*)c->counts.p,
                     sw ? (S1WinDesc*)c->wdesc.p : nullptr, (SlotDesc*)c->slots.p, c->sm_count, c->stream, band,
-                    tiles ? kPlanTiles : kPlanSlots);
+                    tiles ? kPlanTiles : kPlanSlots, windows ? (WinGroup*)c->groups.p : nullptr);
         launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
                         scan_u64_tmp_elems(slots), c->stream);
         launches += 5;
@@ -1034,6 +1189,21 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         int per_sm = 0;
         sums_kernel_occupancy(256, &per_sm);
         const int grid = c->sm_count * std::max(1, per_sm);
+        if (windows) {
+            TileWinArgs wa;
+            wa.items = (const TileWinItem*)c->titems.p;
+            wa.tasks = (const TileWinTask*)((const char*)c->titems.p + item_bytes);
+            wa.n_tasks = ww.tasks.size();
+            wa.groups = (const WinGroup*)c->groups.p;
+            wa.slots = sa.slots;
+            wa.queries = sa.queries;
+            wa.T = T;
+            wa.rcp = sa.rcp;
+            wa.ticket = sa.ticket + 2;
+            wa.acc = sa.acc;
+            launch_windows(wa, c->sm_count, c->stream);
+            launches += 1;
+        }
         if (tiles) {
             launch_tiles(sa, c->sm_count, c->stream);
             launches += 1;
@@ -1132,6 +1302,7 @@ void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, 
     if (c->graphs.size() >= 4) {
         if (c->graphs.front().exec) cudaGraphExecDestroy(c->graphs.front().exec);
         if (c->graphs.front().stage) cudaFreeHost(c->graphs.front().stage);
+        if (c->graphs.front().tstage) cudaFreeHost(c->graphs.front().tstage);
         c->graphs.erase(c->graphs.begin());
     }
     dr_ctx::Graph g;
@@ -1143,8 +1314,15 @@ void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, 
         cudaGetLastError();
         return;
     }
-    uint8_t* saved = c->stage;
-    const size_t saved_cap = c->stage_cap, saved_used = c->stage_used;
+    if (c->tstage_used && cudaMallocHost((void**)&g.tstage, c->tstage_used) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFreeHost(g.stage);
+        return;
+    }
+    uint8_t *saved = c->stage, *tsaved = c->tstage;
+    const size_t saved_cap = c->stage_cap, saved_used = c->stage_used, tsaved_cap = c->tstage_cap;
+    c->tstage = g.tstage;
+    c->tstage_cap = c->tstage_used;
     c->stage = g.stage;
     c->stage_cap = need;
     c->stage_used = 0;
@@ -1161,11 +1339,14 @@ void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, 
     c->stage = saved;
     c->stage_cap = saved_cap;
     c->stage_used = saved_used;
+    c->tstage = tsaved;
+    c->tstage_cap = tsaved_cap;
     if (rc == DR_OK && graph && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess) {
         g.launches = launches + 3;
         c->graphs.push_back(std::move(g));
     } else {
         if (g.stage) cudaFreeHost(g.stage);
+        if (g.tstage) cudaFreeHost(g.tstage);
     }
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
@@ -1257,12 +1438,13 @@ int dr_ctx_destroy(dr_ctx* c) {
     DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->primes, &c->pinv, &c->items, &c->stencil,
                       &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->counts, &c->ticket, &c->misc,
                       &c->inv, &c->invw, &c->wdesc, &c->witems, &c->slots, &c->prcp, &c->sq_cnt, &c->sq_off, &c->sq_cur,
-                      &c->sq_pos, &c->sq_tmp, &c->items_odd, &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt};
+                      &c->sq_pos, &c->sq_tmp, &c->items_odd, &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->groups, &c->titems};
     for (DevBuf* b : bufs) release(c, *b);
     drop_graphs(c);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->stage) cudaFreeHost(c->stage);
     if (c->wstage) cudaFreeHost(c->wstage);
+    if (c->tstage) cudaFreeHost(c->tstage);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
     for (auto& e : c->bev) cudaEventDestroy(e);
@@ -1477,7 +1659,7 @@ int dr_mertens_batch(dr_ctx* c, const int64_t* X, int64_t count, const dr_params
         if (!rc) break;
     }
     if (rc) return rc;
-    rc = finish_queries(c, X, count, launches, c->stage_used + c->wstage_used, out, st);
+    rc = finish_queries(c, X, count, launches, c->stage_used + c->wstage_used + c->tstage_used, out, st);
     if (rc) return rc;
     if (st) st->total_ms = now_ms() - t0;
     if (count > 1 && c->graphs_enabled) capture_graph(c, X, P.data(), count, tune, ut, ud, ml, n_primes);

@@ -1010,7 +1010,7 @@ __device__ __forceinline__ int query_of_block(const QueryDev* q, int nq, u64 b) 
 __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const TableView T, u64 n_blocks,
                             u64* __restrict__ ops, u64* __restrict__ acc, i64* __restrict__ counts,
                             S1WinDesc* __restrict__ wdesc, SlotDesc* __restrict__ slots, const S1Band band,
-                            const int mode) {
+                            const int mode, WinGroup* __restrict__ groups) {
     const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
     const int lane = threadIdx.x & 31;
     for (u64 w = (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < 2 * n_blocks; w += warps) {
@@ -1022,9 +1022,10 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
         const bool valid = cand < Q.nc;
         const u64 s = Q.slot_base + 2 * (u64)cand + (u64)e;
         u64 v[7] = {0, 0, 0, 0, 0, 0, 0};  // C, terms, evaluations, S1, S2, compressed S1, S1 sum
-        u64 bits = 0;
+        bool tile = false;
+        EvalDesc d;
+        d.kind = EVAL_NONE;
         if (valid) {
-            EvalDesc d;
             decode_eval(Q, T, cand, e, d, band);
             if (band.s1_only && d.kind != EVAL_NONE && d.total <= kBandInThread) {
                 // a band pass: nearly every evaluation has a handful of lookups in the band;
@@ -1041,8 +1042,8 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
                 for (int g = 0; g < kS1Seg; ++g) d.s1_cnt[g] = 0;
                 d.total = 0;
             }
-            const bool tile = mode != kPlanSlots && tile_eligible(d, Q.inv_limit);
-            bits = pack_slot(d, slots + s, tile && mode == kPlanTiles ? kSlotTile : 0ull);
+            tile = mode != kPlanSlots && tile_eligible(d, Q.inv_limit);
+            if (mode != kPlanTiles) pack_slot(d, slots + s, 0ull);
             if (mode == kPlanSlots || mode == kPlanRest) ops[s] = tile ? 0ull : d.total;
             if (wdesc && Q.win) {
                 S1WinDesc wd;
@@ -1077,14 +1078,56 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
         }
         if (mode == kPlanTiles) {
             // the block's groups: one, or a few where the block straddles a range boundary
-            u64 units = 0;
+            u64 sig = 0;
+            if (tile) {
+                sig = kSlotTile | (u64)d.kind;
+                for (int g = 0; g < kS1Seg; ++g) sig |= stride_code(d.s1_stride[g]) << (3 + 3 * g);
+            }
+            unsigned left = __ballot_sync(0xffffffffu, tile);
+            const u64 sig0 = __shfl_sync(0xffffffffu, sig, left ? __ffs(left) - 1 : 0);
+            // the block's windows: its lookups with q < wc * kTileWin are the window kernel's
+            const u64 wc = groups && left && __all_sync(0xffffffffu, !tile || sig == sig0)
+                               ? tile_windows(Q.X, blk, Q.twin_max) : 0;
+            uint32_t near[kS1Seg] = {0u, 0u, 0u, 0u};
             SlotDesc t = {};
-            if (bits & kSlotTile) t = slots[s];
-            unsigned left = __ballot_sync(0xffffffffu, (bits & kSlotTile) != 0);
+            if (tile) {
+                if (wc) {
+                    const i64 ncut = (i64)udiv(d.y, wc * kTileWin) + 1;  // n >= ncut <=> q < wc*kTileWin
+                    for (int g = 0; g < kS1Seg; ++g) {
+                        const i64 cnt = d.s1_cnt[g], n0 = d.s1_n0[g];
+                        if (cnt <= 0) continue;
+                        const int st = d.s1_stride[g];
+                        const i64 far = ncut <= 1 ? 0
+                                        : st == S1_WHEEL ? wheel_upper(ncut - 1) - n0 + 1
+                                        : ncut <= n0 ? 0 : (ncut - 1 - n0) / st + 1;
+                        d.s1_cnt[g] = min(cnt, max((i64)0, far));
+                        near[g] = (uint32_t)(cnt - d.s1_cnt[g]);
+                    }
+                }
+                pack_slot(d, &t, kSlotTile, near);
+            }
+            if (valid) slots[s] = t;
+            if (groups) {
+                WinGroup G = {};
+                G.mm = left;
+                G.wc = (uint32_t)wc;
+                G.bits = (uint32_t)sig0;
+                if (wc) {
+#pragma unroll
+                    for (int g = 0; g < kS1Seg; ++g) {
+                        uint32_t lo = 1, hi = 0, res;
+                        if (tile) win_range(t, g, &lo, &hi, &res);
+                        G.ulo[g] = __reduce_min_sync(0xffffffffu, lo <= hi ? lo : 0xffffffffu);
+                        G.uhi[g] = __reduce_max_sync(0xffffffffu, lo <= hi ? hi : 0u);
+                    }
+                }
+                if (lane == 0) groups[w] = G;
+            }
+            u64 units = 0;
             while (left) {
                 const int lead = __ffs(left) - 1;
-                const u64 sig = __shfl_sync(0xffffffffu, bits & (kSlotTile | kTileSig), lead);
-                const bool member = (bits & (kSlotTile | kTileSig)) == sig;
+                const u64 lead_sig = __shfl_sync(0xffffffffu, sig, lead);
+                const bool member = tile && sig == lead_sig;
                 left &= ~__ballot_sync(0xffffffffu, member);
                 uint32_t sum = 0;
 #pragma unroll
@@ -1114,10 +1157,11 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
 }
 
 void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc, i64* counts,
-                 S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s, const S1Band& band, int mode) {
+                 S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s, const S1Band& band, int mode,
+                 WinGroup* groups) {
     if (n_blocks == 0) return;
     const int grid = (int)std::min<u64>((2 * n_blocks + 3) / 4, (u64)sm_count * 16);
-    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode);
+    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode, groups);
 }
 
 // Direct answers for queries with X <= table u_total (get_M, :1465-1467).

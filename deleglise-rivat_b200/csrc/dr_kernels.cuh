@@ -165,12 +165,36 @@ constexpr int kBandInThread = 64;
 enum { kPlanSlots = 0, kPlanTiles = 1, kPlanRest = 2 };
 void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc,
                  i64* counts, S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s,
-                 const S1Band& band, int mode);
+                 const S1Band& band, int mode, WinGroup* groups = nullptr);
 // Windowed S1 (window length win: a power of two, 2^12 .. 2^16).
 void launch_s1win(const S1WinArgs& a, u64 win, int sm_count, cudaStream_t s);
 void launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t tmp_elems, cudaStream_t s);
 size_t scan_u64_tmp_elems(u64 n);
 void launch_sums(const SumsArgs& a, int grid, int block, cudaStream_t s);
+// Work of the window kernel (dr_windows.cu).  A task, one CTA's: the items [i0, i1) of window
+// w.  An item: the blocks [b0, b1) of query q (counted over the launch's blocks), two groups
+// each, every group in `parts` pieces; its units -- (group, piece), drawn by the CTA's warps
+// -- are numbered from u0 within the task.
+struct TileWinItem {
+    uint32_t b0, b1, q, parts, u0;
+};
+struct TileWinTask {
+    uint32_t w, i0, i1, units;
+};
+struct TileWinArgs {
+    const TileWinItem* items;
+    const TileWinTask* tasks;
+    u64 n_tasks;
+    const WinGroup* groups;  // [2 * blocks]: evaluation 0 and 1 of each block
+    const SlotDesc* slots;
+    const QueryDev* queries;
+    TableView T;
+    const double* rcp;
+    u64* ticket;
+    u64* acc;
+};
+// The S1 lookups below each block's last window, on the groups of a kPlanTiles pass.
+void launch_windows(const TileWinArgs& a, int sm_count, cudaStream_t s);
 // The tile kernel (dr_tiles.cu) on the ops of a kPlanTiles pass.
 void launch_tiles(const SumsArgs& a, int sm_count, cudaStream_t s);
 // Reciprocal tables shared by every evaluation of a launch.

@@ -48,10 +48,6 @@ struct TileWarp {
     double rcp[kTileN];
 };
 
-__device__ __forceinline__ uint32_t floor_q(double yd, double r) {
-    return (uint32_t)__double2loint(__fma_rd(yd, r, kTwo52));
-}
-
 // exact double of a 32-bit integer on the FP64 pipe (the conversions run on a narrower one)
 __device__ __forceinline__ double u32_double(uint32_t v) {
     return __hiloint2double(0x43300000, (int)v) - kTwo52;
@@ -73,11 +69,6 @@ __device__ __forceinline__ u64 warp_upper_slot(const u64* prefix, u64 n_slots, u
         lo = base;
     }
     return lo;
-}
-
-// divisor of index i in an S1 segment of stride code `code` (1, 2, 6, wheel)
-__device__ __forceinline__ uint32_t tile_n(uint32_t code, uint32_t i, uint32_t res) {
-    return code == 0 ? i : code == 1 ? 2u * i + res : code == 2 ? 6u * i + res : 3u * i + 1u + (i & 1u);
 }
 
 // S1, lanes on divisors: 4 divisors per lane, members one after another, every quotient in
@@ -359,8 +350,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
                     const uint32_t code = (kbits >> (3 + 3 * g)) & 3u;
                     res = __reduce_max_sync(0xffffffffu, some ? res : 0u);
                     const double span = code == 0 ? 32.0 : code == 1 ? 64.0 : code == 2 ? 192.0 : 96.0;
-                    for (u64 u = a0; u < a1; ++u) {
-                        const uint32_t i0 = ulo + kTileN * (uint32_t)(u - ub), i1 = i0 + (kTileN - 1);
+                    // blocks whose first unit is the ticket's
+                    const uint32_t b0 = ((uint32_t)(a0 - ub) + kTileS1Units - 1u) / kTileS1Units;
+                    const uint32_t b1 = ((uint32_t)(a1 - ub) + kTileS1Units - 1u) / kTileS1Units;
+                    for (uint32_t blk = b0; blk < b1; ++blk) {
+                        const uint32_t i0 = ulo + kTileN * blk, i1 = i0 + (kTileN - 1);
                         const unsigned act = __ballot_sync(0xffffffffu, some && lo <= i1 && hi >= i0);
                         const unsigned whole = __ballot_sync(0xffffffffu, some && lo <= i0 && hi >= i1);
                         if (act == 0) continue;
