@@ -77,8 +77,9 @@ struct dr_ctx {
     uint64_t budget = 0;
     uint64_t held = 0;
     // table buffers
-    DevBuf dM, planes, ckpt, wheel, seg_sum, seg_off, primes, pinv, items, stencil, prcp;
-    DevBuf items_odd, stencil_odd, dplanes;  // odd-mode sieve: items, stencil, dense-tier plane words
+    DevBuf dM, planes, ckpt, wheel, seg_sum, seg_off, stencil;
+    DevBuf consts;                // sieving primes, their reciprocals and the work items (upload_consts)
+    DevBuf stencil_odd, dplanes;  // odd-mode sieve: stencil, dense-tier plane words
     DevBuf sq_cnt, sq_off, sq_cur, sq_pos, sq_tmp;  // bucketed square hits per segment
     // streamed table (dr_ctx_set_resident_limit): above u_resident the compressed tier
     // is built and consumed band by band in these two buffers, never held whole
@@ -87,7 +88,8 @@ struct dr_ctx {
     std::vector<cudaEvent_t> bev;  // band timing: start, then per band after its build and after its sums
     int64_t last_bands = 0;        // bands the enqueued call streams
     // query buffers
-    DevBuf queries, ops, prefix, scan_tmp, acc, counts, ticket, misc, inv, invw, wdesc, witems, slots;
+    DevBuf queries, ops, prefix, scan_tmp, misc, inv, invw, wdesc, witems, slots;
+    DevBuf acc;             // results: 3 sums and kCountsPerQuery counters per query, then 4 words of work queues
     DevBuf groups, titems;  // window kernel: tile groups; work items and tasks
     // table state
     bool table_valid = false;
@@ -108,7 +110,8 @@ struct dr_ctx {
     static constexpr int kForks = 40;
     cudaEvent_t fork[kForks] = {};
     cudaEvent_t join = nullptr;
-    bool sieve_attr_set = false;
+    // launch shapes found once: CTAs per SM of the sieve (last shape), sums and tile kernels
+    int sv_S = 0, sv_block = 0, sv_full = 0, sv_odd = 0, sums_per_sm = 0, tiles_per_sm = 0;
     // pinned staging for every host->device source of a call (a captured graph
     // owns its own staging, so replays never read memory a later call reuses)
     uint8_t* stage = nullptr;
@@ -189,10 +192,9 @@ bool release_scratch(dr_ctx* c) {
     cudaStreamSynchronize(c->side);
     cudaGetLastError();
     drop_graphs(c);
-    DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->primes, &c->pinv,
-                      &c->items, &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->counts, &c->ticket,
-                      &c->misc, &c->inv, &c->invw, &c->wdesc, &c->witems, &c->slots, &c->prcp, &c->sq_cnt,
-                      &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp, &c->items_odd, &c->dplanes, &c->bplanes,
+    DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->consts, &c->queries,
+                      &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->misc, &c->inv, &c->invw, &c->wdesc, &c->witems,
+                      &c->slots, &c->sq_cnt, &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp, &c->dplanes, &c->bplanes,
                       &c->bckpt, &c->groups, &c->titems};
     bool any = false;
     for (DevBuf* b : bufs) {
@@ -272,6 +274,8 @@ const std::vector<uint32_t>& primes_upto(dr_ctx* c, int64_t root) {
         c->host_pinv[i] = ~0ull / p;
         c->host_pinv[np + i] = ~0ull / (p * p);
     }
+    c->host_prcp.resize(np);
+    for (size_t i = 0; i < np; ++i) c->host_prcp[i] = 1.0 / (double)c->host_primes[i];  // IEEE: RN(1/p)
     return c->host_primes;
 }
 
@@ -332,28 +336,75 @@ int check_table_limits(int64_t u_total, int64_t u_dense, int64_t mu_limit) {
     return DR_OK;
 }
 
-// The sieve's moduli for B sieved bytes per segment (S in full mode, S/2 in odd mode):
-// warp items for the moduli below B/kItemDiv (uploaded into buf), one thread per prime
-// above.  m.w_first and m.sq_first must be set.
-int set_sieve_moduli(dr_ctx* c, const std::vector<uint32_t>& pr, int B, SieveArgs& m, DevBuf& buf) {
-    m.tierB_first = std::max(m.w_first, (int)(std::lower_bound(pr.begin(), pr.end(),
-                                                                (uint32_t)std::max(13, B / kItemDiv)) - pr.begin()));
-    int k = m.sq_first;  // first prime whose square reaches B/kItemDiv
+// The sieve's moduli for B sieved bytes per segment (S in full mode, S/2 in odd mode): warp
+// items for the moduli below B/kItemDiv, one thread per prime above.
+struct Moduli {
+    int tierB_first = 0, sqB_first = 0, n_items = 0;
+    std::vector<uint4> items;
+    void set(SieveArgs& a, const uint4* dev) const {
+        a.tierB_first = tierB_first;
+        a.sqB_first = sqB_first;
+        a.n_items = n_items;
+        a.items = dev;
+    }
+};
+
+int sieve_moduli(const std::vector<uint32_t>& pr, int B, int w_first, int sq_first, Moduli& m) {
+    m.tierB_first = std::max(w_first, (int)(std::lower_bound(pr.begin(), pr.end(),
+                                                              (uint32_t)std::max(13, B / kItemDiv)) - pr.begin()));
+    int k = sq_first;  // first prime whose square reaches B/kItemDiv
     while (k < (int)pr.size() && (uint64_t)pr[k] * pr[k] < (uint64_t)(B / kItemDiv)) ++k;
     m.sqB_first = k;
-    std::vector<uint4> items(kMaxSieveItems);
-    m.n_items = build_sieve_items(pr.data(), (int)pr.size(), B, items.data(), kMaxSieveItems);
+    m.items.resize(kMaxSieveItems);
+    m.n_items = build_sieve_items(pr.data(), (int)pr.size(), B, m.items.data(), kMaxSieveItems);
     if (m.n_items < 0) return fail(DR_ERR_PARAMS, "sieve work items exceed %d for %d bytes per segment", kMaxSieveItems, B);
-    int e = ensure(c, buf, (size_t)std::max(m.n_items, 1) * 16);
-    if (e) return e;
-    if (m.n_items) {
-        const void* si = stage_put(c, items.data(), (size_t)m.n_items * 16);
-        if (!si) return fail(DR_ERR_NOMEM, "internal: staging area too small");
-        if (cudaMemcpyAsync(buf.p, si, (size_t)m.n_items * 16, cudaMemcpyHostToDevice, c->stream) != cudaSuccess)
-            return fail(DR_ERR_CUDA, "sieve items upload failed");
-    }
-    m.items = (const uint4*)buf.p;
     return DR_OK;
+}
+
+size_t consts_bytes(size_t np, int items) { return np * 28 + (size_t)items * 16 + 64; }
+
+// The primes, their reciprocals and the work items of the full mode (moduli f, into a) and of
+// the odd mode (moduli o, into ao; both NULL where it is not used): one device buffer, one copy.
+int upload_consts(dr_ctx* c, const std::vector<uint32_t>& pr, const Moduli& f, const Moduli* o, SieveArgs& a,
+                  SieveArgs* ao) {
+    const size_t np = pr.size(), n_odd = o ? (size_t)o->n_items : 0;
+    const size_t at_inv = (np * 4 + 15) & ~size_t(15), at_rcp = at_inv + np * 16;
+    const size_t at_items = (at_rcp + np * 8 + 15) & ~size_t(15), at_odd = at_items + (size_t)f.n_items * 16;
+    const size_t total = at_odd + n_odd * 16, at = (c->stage_used + 15) & ~size_t(15);
+    int rc = ensure(c, c->consts, total);
+    if (rc) return rc;
+    if (at + total > c->stage_cap) return fail(DR_ERR_NOMEM, "internal: staging area too small");
+    uint8_t* h = c->stage + at;
+    std::memcpy(h, pr.data(), np * 4);
+    std::memcpy(h + at_inv, c->host_pinv.data(), np * 16);
+    std::memcpy(h + at_rcp, c->host_prcp.data(), np * 8);
+    std::memcpy(h + at_items, f.items.data(), (size_t)f.n_items * 16);
+    if (o) std::memcpy(h + at_odd, o->items.data(), n_odd * 16);
+    c->stage_used = at + total;
+    if (total) CU(cudaMemcpyAsync(c->consts.p, h, total, cudaMemcpyHostToDevice, c->stream));
+    const uint8_t* d = (const uint8_t*)c->consts.p;
+    a.primes = (const uint32_t*)d;
+    a.pinv = (const u64*)(d + at_inv);
+    a.sqinv = a.pinv + np;
+    a.prcp = (const double*)(d + at_rcp);
+    f.set(a, (const uint4*)(d + at_items));
+    if (ao) {
+        *ao = a;
+        o->set(*ao, (const uint4*)(d + at_odd));
+    }
+    return DR_OK;
+}
+
+// CTAs per SM of the sieve for a shape.
+void sieve_occupancy(dr_ctx* c, int S, int block, int* full, int* odd) {
+    if (c->sv_S != S || c->sv_block != block) {
+        sieve_kernel_attrs(sieve_smem_bytes(S, false), false, block, &c->sv_full);
+        sieve_kernel_attrs(sieve_smem_bytes(S, true), true, block, &c->sv_odd);
+        c->sv_S = S;
+        c->sv_block = block;
+    }
+    *full = c->sv_full;
+    *odd = c->sv_odd;
 }
 
 int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, const dr_params* tuning,
@@ -381,23 +432,6 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     if ((rc = ensure(c, c->seg_sum, (size_t)nseg * 4))) return rc;
     if ((rc = ensure(c, c->seg_off, (size_t)(nseg + 1) * 4))) return rc;
     const std::vector<uint32_t>& pr = primes_upto(c, isqrt_i64(u_total));
-    if ((rc = ensure(c, c->primes, pr.size() * 4))) return rc;
-    if ((rc = ensure(c, c->pinv, pr.size() * 16))) return rc;
-    if ((rc = ensure(c, c->prcp, pr.size() * 8))) return rc;
-    if (c->host_prcp.size() != pr.size()) {
-        c->host_prcp.resize(pr.size());
-        for (size_t i = 0; i < pr.size(); ++i) c->host_prcp[i] = 1.0 / (double)pr[i];  // IEEE: RN(1/p)
-    }
-    if (!pr.empty()) {
-        const void* sp = stage_put(c, pr.data(), pr.size() * 4);
-        const void* sv = stage_put(c, c->host_pinv.data(), pr.size() * 16);
-        const void* sr = stage_put(c, c->host_prcp.data(), pr.size() * 8);
-        if (!sp || !sv || !sr) return fail(DR_ERR_NOMEM, "internal: staging area too small");
-        CU(cudaMemcpyAsync(c->primes.p, sp, pr.size() * 4, cudaMemcpyHostToDevice, c->stream));
-        CU(cudaMemcpyAsync(c->pinv.p, sv, pr.size() * 16, cudaMemcpyHostToDevice, c->stream));
-        CU(cudaMemcpyAsync(c->prcp.p, sr, pr.size() * 8, cudaMemcpyHostToDevice, c->stream));
-    }
-
     SieveArgs a;
     a.u_total = u_total;
     a.u_dense = u_dense;
@@ -412,17 +446,24 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     };
     a.sq_first = first_at_least(5);
     a.w_first = first_at_least(13);
-    auto set_moduli = [&](SieveArgs& m, int B, DevBuf& buf) { return set_sieve_moduli(c, pr, B, m, buf); };
-    if ((rc = set_moduli(a, a.S_sub, c->items))) return rc;
-    a.primes = (const uint32_t*)c->primes.p;
-    a.pinv = (const u64*)c->pinv.p;
-    a.sqinv = (const u64*)c->pinv.p + pr.size();
-    a.prcp = (const double*)c->prcp.p;
+    // Launch plan: the first wave of segments in full mode, the rest in odd mode,
+    // in launches [b0, b1) whose halves lie below b0 (ranges roughly doubling).
+    const size_t smem_f = sieve_smem_bytes(S, false), smem_o = sieve_smem_bytes(S, true);
+    int per_f = 0, per_o = 0;
+    sieve_occupancy(c, S, block, &per_f, &per_o);
+    const int64_t grid_f = (int64_t)c->sm_count * std::max(per_f, 1);
+    const int64_t grid_o = (int64_t)c->sm_count * std::max(per_o, 1);
+    const std::vector<SieveLaunch> plan = sieve_launch_plan(u_total, u_dense, S, grid_f);
+    bool odd = false;
+    for (const SieveLaunch& l : plan) odd = odd || l.odd;
+    Moduli mf, mo;
+    if ((rc = sieve_moduli(pr, a.S_sub, a.w_first, a.sq_first, mf))) return rc;
+    if (odd && (rc = sieve_moduli(pr, S / 2, a.w_first, a.sq_first, mo))) return rc;
     // squares above S hit a segment at most once: bucket their hits per segment
     // (sizes known here exactly: sum of floor(u_total / p^2) over those primes)
     int lgS = 0;
     while ((1 << lgS) < S) ++lgS;
-    a.sqC_first = a.sqB_first;
+    a.sqC_first = mf.sqB_first;
     while (a.sqC_first < (int)pr.size() && (uint64_t)pr[a.sqC_first] * pr[a.sqC_first] <= (uint64_t)S) ++a.sqC_first;
     uint64_t sq_hits = 0;
     for (size_t i = (size_t)a.sqC_first; i < pr.size(); ++i) sq_hits += (uint64_t)u_total / ((uint64_t)pr[i] * pr[i]);
@@ -452,24 +493,12 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     a.seg_sum = (int32_t*)c->seg_sum.p;
     a.dplanes = nullptr;
 
-    // Launch plan: the first wave of segments in full mode, the rest in odd mode,
-    // in launches [b0, b1) whose halves lie below b0 (ranges roughly doubling).
-    const size_t smem_f = sieve_smem_bytes(S, false), smem_o = sieve_smem_bytes(S, true);
-    int per_f = 0, per_o = 0;
-    sieve_kernel_attrs(smem_f, false, block, &per_f);
-    sieve_kernel_attrs(smem_o, true, block, &per_o);
-    const int64_t grid_f = (int64_t)c->sm_count * std::max(per_f, 1);
-    const int64_t grid_o = (int64_t)c->sm_count * std::max(per_o, 1);
-    const std::vector<SieveLaunch> plan = sieve_launch_plan(u_total, u_dense, S, grid_f);
-    bool odd = false;
-    for (const SieveLaunch& l : plan) odd = odd || l.odd;
-    SieveArgs ao = a;
     if (odd) {
         if ((rc = ensure(c, c->dplanes, (size_t)(u_dense / 64 + 1) * 16))) return rc;
         a.dplanes = (ulonglong2*)c->dplanes.p;
-        ao = a;
-        if ((rc = set_moduli(ao, S / 2, c->items_odd))) return rc;
     }
+    SieveArgs ao;
+    if ((rc = upload_consts(c, pr, mf, odd ? &mo : nullptr, a, odd ? &ao : nullptr))) return rc;
 
     CU(record_event(c, 0));
     CU(cudaMemsetAsync(c->wheel.p, 0, (size_t)wheel_groups * 16, c->stream));
@@ -477,11 +506,11 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     if (a.sq_off) {
         CU(cudaMemsetAsync(c->sq_cnt.p, 0, (size_t)nseg * 8, c->stream));
         CU(cudaMemsetAsync(c->sq_cur.p, 0, (size_t)nseg * 8, c->stream));
-        launch_sq_bucket_count((const uint32_t*)c->primes.p, a.sqC_first, (int)pr.size(), 0, u_total, u_dense,
+        launch_sq_bucket_count(a.primes, a.sqC_first, (int)pr.size(), 0, u_total, u_dense,
                                dense_segs, lgS, 0, (u64*)c->sq_cnt.p, c->stream);
         launch_scan_u64((const u64*)c->sq_cnt.p, (u64*)c->sq_off.p, (u64)nseg, (u64*)c->sq_tmp.p,
                         scan_u64_tmp_elems((u64)nseg), c->stream);
-        launch_sq_bucket_fill((const uint32_t*)c->primes.p, a.sqC_first, (int)pr.size(), 0, u_total, u_dense,
+        launch_sq_bucket_fill(a.primes, a.sqC_first, (int)pr.size(), 0, u_total, u_dense,
                               dense_segs, lgS, 0, (const u64*)c->sq_off.p, (u64*)c->sq_cur.p, (uint32_t*)c->sq_pos.p,
                               c->stream);
         CU(cudaGetLastError());
@@ -757,11 +786,7 @@ int plan_stream(dr_ctx* c, int64_t X, int64_t ut, int64_t ud, int64_t ml, const 
     int rc;
     if ((rc = ensure(c, c->seg_sum, (size_t)sp->nseg * 4))) return rc;
     if ((rc = ensure(c, c->seg_off, (size_t)(sp->nseg + 1) * 4))) return rc;
-    if ((rc = ensure(c, c->primes, np * 4))) return rc;
-    if ((rc = ensure(c, c->pinv, np * 16))) return rc;
-    if ((rc = ensure(c, c->prcp, np * 8))) return rc;
-    if ((rc = ensure(c, c->items, (size_t)kMaxSieveItems * 16))) return rc;
-    if ((rc = ensure(c, c->items_odd, (size_t)kMaxSieveItems * 16))) return rc;
+    if ((rc = ensure(c, c->consts, consts_bytes(np, 2 * kMaxSieveItems)))) return rc;
     if ((rc = ensure(c, c->bplanes, bwords * 16))) return rc;
     if ((rc = ensure(c, c->bckpt, bwords * 4))) return rc;
     if (max_sq > 0) {
@@ -781,15 +806,6 @@ int plan_stream(dr_ctx* c, int64_t X, int64_t ut, int64_t ud, int64_t ml, const 
 int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid, int* launches) {
     const std::vector<uint32_t>& pr = primes_upto(c, isqrt_i64(sp.u_total));
     const size_t np = pr.size();
-    std::vector<double> prcp(np);
-    for (size_t i = 0; i < np; ++i) prcp[i] = 1.0 / (double)pr[i];  // IEEE: RN(1/p)
-    const void* sp_ = stage_put(c, pr.data(), np * 4);
-    const void* sv = stage_put(c, c->host_pinv.data(), np * 16);
-    const void* sr = stage_put(c, prcp.data(), np * 8);
-    if (!sp_ || !sv || !sr) return fail(DR_ERR_NOMEM, "internal: staging area too small");
-    CU(cudaMemcpyAsync(c->primes.p, sp_, np * 4, cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->pinv.p, sv, np * 16, cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemcpyAsync(c->prcp.p, sr, np * 8, cudaMemcpyHostToDevice, c->stream));
     const int S = sp.S;
     int lgS = 0;
     while ((1 << lgS) < S) ++lgS;
@@ -804,13 +820,12 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
     a.n_primes = (int)np;
     a.sq_first = (int)(std::lower_bound(pr.begin(), pr.end(), 5u) - pr.begin());
     a.w_first = (int)(std::lower_bound(pr.begin(), pr.end(), 13u) - pr.begin());
-    int rc = set_sieve_moduli(c, pr, a.S_sub, a, c->items);
+    Moduli mf, mo;  // odd mode: the bands whose halves are resident (band_odd)
+    const bool odd_ok = sp.u_dense % 64 == 0;
+    int rc = sieve_moduli(pr, a.S_sub, a.w_first, a.sq_first, mf);
+    if (!rc && odd_ok) rc = sieve_moduli(pr, S / 2, a.w_first, a.sq_first, mo);
     if (rc) return rc;
-    a.primes = (const uint32_t*)c->primes.p;
-    a.pinv = (const u64*)c->pinv.p;
-    a.sqinv = (const u64*)c->pinv.p + np;
-    a.prcp = (const double*)c->prcp.p;
-    const int sqC = std::max(sp.sqC_first, a.sqB_first);  // squares above S: bucketed per band
+    const int sqC = std::max(sp.sqC_first, mf.sqB_first);  // squares above S: bucketed per band
     a.sq_off = nullptr;
     a.sq_seg0 = 0;
     a.sq_pos = nullptr;
@@ -825,14 +840,11 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
     a.seg_sum = (int32_t*)c->seg_sum.p;
     const size_t smem = sieve_smem_bytes(S, false), smem_o = sieve_smem_bytes(S, true);
     int per = 0, per_o = 0;
-    sieve_kernel_attrs(smem, false, sp.block, &per);
-    sieve_kernel_attrs(smem_o, true, sp.block, &per_o);
+    sieve_occupancy(c, S, sp.block, &per, &per_o);
     const int64_t sgrid = (int64_t)c->sm_count * std::max(per, 1);
     const int64_t sgrid_o = (int64_t)c->sm_count * std::max(per_o, 1);
-    // odd-mode arguments for the bands whose halves are resident (band_odd)
-    SieveArgs ao = a;
-    const bool odd_ok = sp.u_dense % 64 == 0;
-    if (odd_ok && (rc = set_sieve_moduli(c, pr, S / 2, ao, c->items_odd))) return rc;
+    SieveArgs ao;
+    if ((rc = upload_consts(c, pr, mf, odd_ok ? &mo : nullptr, a, odd_ok ? &ao : nullptr))) return rc;
     const int64_t nwords_all = (sp.u_total - sp.u_dense + 63) / 64;
     while ((int64_t)c->bev.size() < 2 * sp.nbands + 1) {
         cudaEvent_t e;
@@ -882,8 +894,8 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
         sa.T.planes = (const ulonglong2*)c->bplanes.p;
         sa.T.ckpt = (const int32_t*)c->bckpt.p;
         sa.T.cbase = cword0;
-        CU(cudaMemsetAsync(c->ticket.p, 0, 8, c->stream));  // the work-queue counter (not the error flag)
-        launch_plan(sa.queries, sa.nq, sa.T, sa.n_blocks, (u64*)c->ops.p, sa.acc, (i64*)c->counts.p, nullptr,
+        CU(cudaMemsetAsync(sa.ticket, 0, 8, c->stream));  // the work-queue counter (not the error flag)
+        launch_plan(sa.queries, sa.nq, sa.T, sa.n_blocks, (u64*)c->ops.p, sa.acc, (i64*)(sa.acc + 3 * sa.nq), nullptr,
                     (SlotDesc*)c->slots.p, c->sm_count, c->stream, S1Band{(u64)vlo + 1, (u64)vhi, 1}, kPlanSlots);
         launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, sa.n_slots, (u64*)c->scan_tmp.p,
                         scan_u64_tmp_elems(sa.n_slots), c->stream);
@@ -1072,13 +1084,15 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     }
     const int64_t invw_count = c->t_mu_limit / 6 + 1;  // every S2 j <= A <= mu_limit
     if ((rc = ensure(c, c->queries, (size_t)nq * sizeof(QueryDev)))) return rc;
-    if ((rc = ensure(c, c->acc, (size_t)nq * 3 * 8))) return rc;
-    if ((rc = ensure(c, c->counts, (size_t)nq * kCountsPerQuery * 8))) return rc;
+    const size_t res_words = (size_t)nq * (3 + kCountsPerQuery) + 4;
+    if ((rc = ensure(c, c->acc, res_words * 8))) return rc;
+    u64* const acc = (u64*)c->acc.p;
+    i64* const counts = (i64*)(acc + 3 * nq);
+    u64* const ticket = acc + (size_t)nq * (3 + kCountsPerQuery);
     if ((rc = ensure(c, c->ops, (size_t)std::max<u64>(slots, 1) * 8))) return rc;
     if ((rc = ensure(c, c->prefix, (size_t)(slots + 1) * 8))) return rc;
     if ((rc = ensure(c, c->slots, (size_t)std::max<u64>(slots, 1) * sizeof(SlotDesc)))) return rc;
     if ((rc = ensure(c, c->scan_tmp, scan_u64_tmp_elems(slots) * 8))) return rc;
-    if ((rc = ensure(c, c->ticket, 32))) return rc;
     if (!witems.empty()) {
         if ((rc = ensure(c, c->wdesc, (size_t)std::max<u64>(slots, 1) * sizeof(S1WinDesc)))) return rc;
         if ((rc = ensure(c, c->witems, witems.size() * sizeof(S1WinItem)))) return rc;
@@ -1135,19 +1149,22 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     const bool tiles = !sw;  // the windowed S1 leaves every other lookup to the sums kernel
     CU(record_event(c, 2));
     CU(cudaMemcpyAsync(c->queries.p, sq, (size_t)nq * sizeof(QueryDev), cudaMemcpyHostToDevice, c->stream));
-    CU(cudaMemsetAsync(c->acc.p, 0, (size_t)nq * 3 * 8, c->stream));
-    CU(cudaMemsetAsync(c->counts.p, 0, (size_t)nq * kCountsPerQuery * 8, c->stream));
-    CU(cudaMemsetAsync(c->ticket.p, 0, 32, c->stream));
+    CU(cudaMemsetAsync(acc, 0, res_words * 8, c->stream));
     if (sw)
         CU(cudaMemcpyAsync(c->witems.p, sw, witems.size() * sizeof(S1WinItem), cudaMemcpyHostToDevice, c->stream));
     if (windows) CU(cudaMemcpyAsync(c->titems.p, c->tstage, c->tstage_used, cudaMemcpyHostToDevice, c->stream));
-    launch_direct((const QueryDev*)c->queries.p, qn, T, (u64*)c->acc.p, c->stream);
-    int launches = 1;
+    int launches = 0;
+    bool direct = false;
+    for (const QueryDev& q : qs) direct = direct || q.N == 0;
+    if (direct) {
+        launch_direct((const QueryDev*)c->queries.p, qn, T, acc, c->stream);
+        launches += 1;
+    }
     if (slots > 0) {
         launch_inverse((double*)c->inv.p, inv_limit, (double2*)c->invw.p, invw_count, T.wheel, c->sm_count,
                        c->stream);
         // a streamed table: this pass takes the S1 lookups with q <= u_res, the bands the rest
-        launch_plan((const QueryDev*)c->queries.p, qn, T, blocks, (u64*)c->ops.p, (u64*)c->acc.p, (i64*)c->counts.p,
+        launch_plan((const QueryDev*)c->queries.p, qn, T, blocks, (u64*)c->ops.p, acc, counts,
                     sw ? (S1WinDesc*)c->wdesc.p : nullptr, (SlotDesc*)c->slots.p, c->sm_count, c->stream, band,
                     tiles ? kPlanTiles : kPlanSlots, windows ? (WinGroup*)c->groups.p : nullptr);
         launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
@@ -1164,8 +1181,8 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         wa.queries = (const QueryDev*)c->queries.p;
         wa.T = T;
         wa.rcp = (const double*)c->inv.p;
-        wa.ticket = (u64*)c->ticket.p + 2;
-        wa.acc = (u64*)c->acc.p;
+        wa.ticket = ticket + 2;
+        wa.acc = acc;
         launch_s1win(wa, qs[0].win, c->sm_count, c->stream);
         CU(cudaGetLastError());
         launches += 1;
@@ -1179,16 +1196,16 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         sa.n_blocks = blocks;
         sa.prefix = (const u64*)c->prefix.p;
         sa.slots = (const SlotDesc*)c->slots.p;
-        sa.ticket = (u64*)c->ticket.p;
-        sa.acc = (u64*)c->acc.p;
+        sa.ticket = ticket;
+        sa.acc = acc;
         sa.chunk_log2 = tuning ? tuning->chunk_log2 : 0;
         sa.rcp = (const double*)c->inv.p;
         sa.inv_limit = inv_limit;
         sa.invw = (const double2*)c->invw.p;
         sa.invw_count = invw_count;
-        int per_sm = 0;
-        sums_kernel_occupancy(256, &per_sm);
-        const int grid = c->sm_count * std::max(1, per_sm);
+        if (!c->sums_per_sm) sums_kernel_occupancy(256, &c->sums_per_sm);
+        if (!c->tiles_per_sm) tiles_kernel_occupancy(&c->tiles_per_sm);
+        const int grid = c->sm_count * std::max(1, c->sums_per_sm);
         if (windows) {
             TileWinArgs wa;
             wa.items = (const TileWinItem*)c->titems.p;
@@ -1205,16 +1222,16 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
             launches += 1;
         }
         if (tiles) {
-            launch_tiles(sa, c->sm_count, c->stream);
+            launch_tiles(sa, c->sm_count * std::max(1, c->tiles_per_sm), c->stream);
             launches += 1;
         }
         if (tiles && rest) {
             // what the tile kernel leaves (y >= 2^51: a few small k of an X above it)
-            launch_plan(sa.queries, qn, T, blocks, (u64*)c->ops.p, sa.acc, (i64*)c->counts.p, nullptr,
+            launch_plan(sa.queries, qn, T, blocks, (u64*)c->ops.p, acc, counts, nullptr,
                         (SlotDesc*)c->slots.p, c->sm_count, c->stream, band, kPlanRest);
             launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
                             scan_u64_tmp_elems(slots), c->stream);
-            CU(cudaMemsetAsync(c->ticket.p, 0, 8, c->stream));  // the work-queue counter (not the error flag)
+            CU(cudaMemsetAsync(ticket, 0, 8, c->stream));  // the work-queue counter (not the error flag)
             launches += 4;
         }
         if (!tiles || rest) {
@@ -1228,11 +1245,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         }
     }
     CU(record_event(c, 4));
-    CU(cudaMemcpyAsync(c->pinned, c->acc.p, (size_t)nq * 3 * 8, cudaMemcpyDeviceToHost, c->stream));
-    CU(cudaMemcpyAsync(c->pinned + (size_t)nq * 3, c->counts.p, (size_t)nq * kCountsPerQuery * 8, cudaMemcpyDeviceToHost,
-                       c->stream));
-    CU(cudaMemcpyAsync(c->pinned + (size_t)nq * (3 + kCountsPerQuery), c->ticket.p, 16, cudaMemcpyDeviceToHost,
-                       c->stream));
+    CU(cudaMemcpyAsync(c->pinned, acc, (res_words - 2) * 8, cudaMemcpyDeviceToHost, c->stream));
     CU(record_event(c, 5));
     *launches_out = launches;
     return DR_OK;
@@ -1435,10 +1448,10 @@ int dr_ctx_destroy(dr_ctx* c) {
     if (!c) return DR_OK;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->primes, &c->pinv, &c->items, &c->stencil,
-                      &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->counts, &c->ticket, &c->misc,
-                      &c->inv, &c->invw, &c->wdesc, &c->witems, &c->slots, &c->prcp, &c->sq_cnt, &c->sq_off, &c->sq_cur,
-                      &c->sq_pos, &c->sq_tmp, &c->items_odd, &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->groups, &c->titems};
+    DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->consts, &c->stencil,
+                      &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->misc, &c->inv, &c->invw, &c->wdesc,
+                      &c->witems, &c->slots, &c->sq_cnt, &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp,
+                      &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->groups, &c->titems};
     for (DevBuf* b : bufs) release(c, *b);
     drop_graphs(c);
     if (c->pinned) cudaFreeHost(c->pinned);

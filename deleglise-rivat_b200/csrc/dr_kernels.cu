@@ -1256,12 +1256,43 @@ __global__ void __launch_bounds__(kScanBlock) scan_tile_apply(const u64* in, u64
     if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = tile_off[ntiles];
 }
 
+// The same scan by one CTA, tile after tile.
+__global__ void __launch_bounds__(kScanBlock) scan_one(const u64* in, u64 n, u64* out) {
+    __shared__ u64 wtot[33];
+    u64 carry = 0;
+    for (u64 b = 0; b < n; b += kScanTile) {
+        const u64 base = b + (u64)threadIdx.x * kScanItems;
+        u64 v[kScanItems];
+        u64 s = 0;
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            v[k] = base + k < n ? in[base + k] : 0;
+            s += v[k];
+        }
+        u64 total;
+        u64 run = carry + block_excl_scan_u64(s, wtot, &total);
+#pragma unroll
+        for (int k = 0; k < kScanItems; ++k) {
+            if (base + k < n) out[base + k] = run;
+            run += v[k];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) out[n] = carry;
+}
+// Tiles up to which one launch beats three (about 2 us a launch).
+constexpr u64 kScanOneTiles = 4;
+
 size_t scan_u64_tmp_elems(u64 n) { return (size_t)((n + kScanTile - 1) / kScanTile) + 1; }
 
 void launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t, cudaStream_t s) {
     const u64 ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles == 0) {
         cudaMemsetAsync(out, 0, sizeof(u64), s);
+        return;
+    }
+    if (ntiles <= kScanOneTiles) {
+        scan_one<<<1, kScanBlock, 0, s>>>(in, n, out);
         return;
     }
     scan_tile_sums<<<(unsigned)ntiles, kScanBlock, 0, s>>>(in, n, tmp);

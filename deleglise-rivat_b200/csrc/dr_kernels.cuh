@@ -196,7 +196,8 @@ struct TileWinArgs {
 // The S1 lookups below each block's last window, on the groups of a kPlanTiles pass.
 void launch_windows(const TileWinArgs& a, int sm_count, cudaStream_t s);
 // The tile kernel (dr_tiles.cu) on the ops of a kPlanTiles pass.
-void launch_tiles(const SumsArgs& a, int sm_count, cudaStream_t s);
+void launch_tiles(const SumsArgs& a, int grid, cudaStream_t s);
+void tiles_kernel_occupancy(int* per_sm);
 // Reciprocal tables shared by every evaluation of a launch.
 void launch_inverse(double* rcp, i64 inv_limit, double2* invw, i64 invw_count, const uint4* wheel, int sm_count,
                     cudaStream_t s);

@@ -269,11 +269,12 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
     const int16_t* dMm1 = a.T.dM - 1;  // dMm1[q] = M(q)
     const double dense_q = (double)min(a.T.u_dense, (i64)0xFFFFFFFEll);
     const u64 total = a.prefix[a.n_slots];
-    // Units per ticket: neighbouring units of a group share table lines in L1 and the set-up
-    // of the group, so up to 32, but 16 tickets per warp so that the last ones do not wait
-    // for one long one (8 tickets: 0.58 against 0.41 ms at M(10^13); 32: 0.47 ms).
+    // Units per ticket: neighbouring units of a group share its set-up and table lines in L1,
+    // so up to 64 (32: 2% more at M(10^16), 4% at the 256-query batch), but 16 tickets per warp
+    // so that the last ones do not wait for one long one (8 tickets of up to 128: 2.0 -> 2.5 ms
+    // at M(2 * 10^14)).
     u64 per = a.chunk_log2 > 0 ? 1ull << max(0, min(a.chunk_log2 - 12, 5)) : 0ull;  // a unit: about 2^12 ops
-    if (per == 0) per = max((u64)1, min(total / ((u64)gridDim.x * kTileWarps * 16), (u64)32));
+    if (per == 0) per = max((u64)4, min(total / ((u64)gridDim.x * kTileWarps * 16), (u64)64));
     int cur_q = -1;
     u64 s1 = 0, s2 = 0;
     for (;;) {
@@ -454,10 +455,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
 
 }  // namespace
 
-void launch_tiles(const SumsArgs& a, int sm_count, cudaStream_t s) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tiles_kernel, 32 * kTileWarps, 0);
-    tiles_kernel<<<sm_count * std::max(1, per_sm), 32 * kTileWarps, 0, s>>>(a);
+void tiles_kernel_occupancy(int* per_sm) {
+    *per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, tiles_kernel, 32 * kTileWarps, 0);
 }
+
+void launch_tiles(const SumsArgs& a, int grid, cudaStream_t s) { tiles_kernel<<<grid, 32 * kTileWarps, 0, s>>>(a); }
 
 }  // namespace drb
