@@ -398,8 +398,8 @@ int upload_consts(dr_ctx* c, const std::vector<uint32_t>& pr, const Moduli& f, c
 // CTAs per SM of the sieve for a shape.
 void sieve_occupancy(dr_ctx* c, int S, int block, int* full, int* odd) {
     if (c->sv_S != S || c->sv_block != block) {
-        sieve_kernel_attrs(sieve_smem_bytes(S, false), false, block, &c->sv_full);
-        sieve_kernel_attrs(sieve_smem_bytes(S, true), true, block, &c->sv_odd);
+        sieve_kernel_attrs(sieve_smem_bytes(S, false), kSieveFull, block, &c->sv_full);
+        sieve_kernel_attrs(sieve_smem_bytes(S, true), kSieveOdd, block, &c->sv_odd);
         c->sv_S = S;
         c->sv_block = block;
     }
@@ -529,7 +529,7 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
         SieveArgs& m = l.odd ? ao : a;
         m.seg_begin = l.begin;
         m.seg_end = l.end;
-        launch_sieve(m, l.odd, (int)std::max<int64_t>(1, std::min<int64_t>(l.end - l.begin, l.odd ? grid_o : grid_f)),
+        launch_sieve(m, l.odd ? kSieveOdd : kSieveFull, (int)std::max<int64_t>(1, std::min<int64_t>(l.end - l.begin, l.odd ? grid_o : grid_f)),
                      block, l.odd ? smem_o : smem_f, c->stream);
         CU(cudaGetLastError());
         if (plan.size() == 1) {  // nothing to overlap: no side stream
@@ -883,7 +883,7 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
         } else {
             m.sqC_first = (int)np;  // no bucketed hit in this band: squares thread-per-prime
         }
-        launch_sieve(m, odd, (int)std::max<int64_t>(1, std::min<int64_t>(c1 - c0, odd ? sgrid_o : sgrid)), sp.block,
+        launch_sieve(m, odd ? kSieveOdd : kSieveFull, (int)std::max<int64_t>(1, std::min<int64_t>(c1 - c0, odd ? sgrid_o : sgrid)), sp.block,
                      odd ? smem_o : smem, c->stream);
         launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, c0, c1, 1024, c->stream);
         launch_fixup_range((int16_t*)c->dM.p, sp.u_dense, S, (const int32_t*)c->seg_off.p, (int32_t*)c->bckpt.p,

@@ -185,6 +185,11 @@ struct FusedFinal {
     uint32_t kbelow, kabove;
 };
 
+//
+// ANY: the segment's base is any value above 2 u_dense (the caller's u_dense need not lie on a
+// 64-value word).  With an odd base the odd values are the odd b, and the 32 values m start
+// anywhere in a plane word: they come from two.
+template <bool ANY>
 __device__ __forceinline__ void planes_odd_mode(const SieveArgs& a, const uint32_t* buf32, int w, int nw16,
                                                 int lane, i64 base, const FusedFinal& fz, u64* nz, u64* neg) {
     const uint32_t rot = (uint32_t)(lane >> 2) & 7u;
@@ -243,6 +248,24 @@ __device__ __forceinline__ void planes_odd_mode(const SieveArgs& a, const uint32
     const uint32_t sh = (8u * rot) & 31u;
     u64 z = ((u64)__funnelshift_l(zl, zh, sh) << 32) | __funnelshift_l(zh, zl, sh);
     u64 g = ((u64)__funnelshift_l(gl, gh, sh) << 32) | __funnelshift_l(gh, gl, sh);
+    if (ANY) {
+        const int par = (int)(base & 1);
+        const i64 m0 = ((base + 2 - par) >> 1) + 32 * (i64)w;  // the m of b = 1 - par
+        const u64 t = (u64)(m0 - 1 - a.u_dense);
+        const uint32_t bit = (uint32_t)t & 63u;
+        const ulonglong2 P = __ldg(a.hplanes + (t >> 6));
+        u64 hz = P.x >> bit, hg = P.y >> bit;
+        if (bit > 32u) {  // the last of the 32 lie in the next word
+            const ulonglong2 N = __ldg(a.hplanes + (t >> 6) + 1);
+            hz |= N.x << (64u - bit);
+            hg |= N.y << (64u - bit);
+        }
+        const uint32_t oddm = (m0 & 1) ? 0x55555555u : 0xAAAAAAAAu;
+        const uint32_t ez = (uint32_t)hz & oddm, eg = (uint32_t)hz & ~(uint32_t)hg & oddm;
+        *nz = (z << par) | (spread32(ez) << (1 - par));
+        *neg = (g << par) | (spread32(eg) << (1 - par));
+        return;
+    }
     const i64 q0 = (base >> 1) + 32 * (i64)w;  // 0-based bit index of m = q0 + 1
     const i64 G = q0 >> 6;
     const ulonglong2 P = G < (a.u_dense >> 6) ? __ldg(a.dplanes + G) : __ldg(a.hplanes + (G - (a.u_dense >> 6)));
@@ -315,8 +338,9 @@ __device__ __forceinline__ void mark_item(uint32_t* buf32, const uint4 I, const 
 // ---------------------------------------------------------------------------
 // Segmented byte-log Mobius sieve + table outputs (ODD: odd values only).
 // ---------------------------------------------------------------------------
-template <bool ODD>
+template <int MODE>
 __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
+    constexpr bool ODD = MODE != kSieveFull, ANY = MODE == kSieveOddAny;
     extern __shared__ __align__(16) unsigned char smem[];
     uint8_t* buf = smem;
     uint32_t* buf32 = reinterpret_cast<uint32_t*>(smem);
@@ -367,7 +391,7 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
             } else {
                 const uint32_t pidx = myI.w & 0x7fffffffu;
                 const u64 inv = (myI.w >> 31) ? __ldg(a.sqinv + pidx) : __ldg(a.pinv + pidx);
-                const u64 v0 = (u64)seg_base + 1 + 2ull * myI.y;  // the odd value of byte I.y
+                const u64 v0 = (u64)seg_base + 1 + (ANY ? (u64)seg_base & 1 : 0) + 2ull * myI.y;  // the odd value of byte I.y
                 const uint32_t r = (uint32_t)umod_inv(v0, m, inv);
                 uint32_t d = r ? m - r : 0u;
                 if (d & 1u) d += m;
@@ -383,9 +407,10 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
       for (i64 base = seg_base; base < seg_end; base += pass_len) {
         const i64 end = min(base + pass_len, seg_end);
         const int len = (int)(end - base);
-        const i64 low = base + 1;
+        const int par = ANY ? (int)(base & 1) : 0;
+        const i64 low = base + 1 + par;
         // sieved bytes: value low + j (full) or the odd value low + 2j (ODD; low is odd)
-        const int nb = ODD ? (len + 1) >> 1 : len;
+        const int nb = ODD ? (len + 1 - par) >> 1 : len;
         const int ng = (nb + 15) >> 4;  // 16-byte groups
         const int nw16 = ng * 4;        // words covering the groups
 
@@ -396,7 +421,7 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
             const uint32_t P = ODD ? (uint32_t)kStencilOddPeriod : (uint32_t)kStencilPeriod;
             const uint32_t* st = ODD ? a.stencil_odd4 : a.stencil4;
             const uint32_t W = ODD ? (uint32_t)kStencilOddWords : (uint32_t)kStencilWords;
-            const i64 p0 = ODD ? base >> 1 : base;
+            const i64 p0 = ODD ? (low - 1) >> 1 : base;
             uint32_t ph = (uint32_t)((p0 + 4 * (i64)tid) % P);
             const uint32_t step = (4u * (uint32_t)T) % P;
             for (int i = tid; i < nw16; i += T) {
@@ -454,7 +479,7 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
                 if (j < off || j - off >= (uint32_t)len) continue;
                 j -= off;
                 if (ODD) {
-                    if (j & 1u) continue;  // even value
+                    if ((j & 1u) != (uint32_t)par) continue;  // even value
                     j >>= 1;
                 }
                 atomicOr(&buf32[j >> 2], 0x80u << ((j & 3) * 8));
@@ -576,7 +601,7 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
             const u64 lastmask = (len & 63) ? (1ull << (len & 63)) - 1 : ~0ull;
             for (int w = tid; w < nwords; w += T) {
                 u64 nz, neg;
-                planes_odd_mode(a, buf32, w, nw16, lane, base, fz, &nz, &neg);
+                planes_odd_mode<ANY>(a, buf32, w, nw16, lane, base, fz, &nz, &neg);
                 if (w == nwords - 1) {
                     nz &= lastmask;
                     neg &= lastmask;
@@ -714,24 +739,25 @@ int sieve_items_prefix(const uint4* items, int n_items, int n_primes) {
     return k;
 }
 
-void sieve_kernel_attrs(size_t smem, bool odd, int block, int* per_sm) {
+namespace {
+typedef void (*SieveFn)(const SieveArgs);
+SieveFn sieve_of(int mode) {
+    return mode == kSieveFull ? sieve_kernel<kSieveFull>
+           : mode == kSieveOdd ? sieve_kernel<kSieveOdd> : sieve_kernel<kSieveOddAny>;
+}
+}  // namespace
+
+void sieve_kernel_attrs(size_t smem, int mode, int block, int* per_sm) {
     *per_sm = 0;
     // the opt-in limit is the kernel's, for every context and shape: always the largest
-    if (odd) {
-        cudaFuncSetAttribute(sieve_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sieve_smem_bytes(1 << 18, true));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sieve_kernel<true>, block, smem);
-    } else {
-        cudaFuncSetAttribute(sieve_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sieve_smem_bytes(1 << 18, false));
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sieve_kernel<false>, block, smem);
-    }
+    cudaFuncSetAttribute(sieve_of(mode), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)sieve_smem_bytes(1 << 18, mode != kSieveFull));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, sieve_of(mode), block, smem);
 }
 
-void launch_sieve(const SieveArgs& a, bool odd, int grid, int block, size_t smem, cudaStream_t s) {
+void launch_sieve(const SieveArgs& a, int mode, int grid, int block, size_t smem, cudaStream_t s) {
     if (a.seg_end <= a.seg_begin) return;
-    if (odd) sieve_kernel<true><<<grid, block, smem, s>>>(a);
-    else sieve_kernel<false><<<grid, block, smem, s>>>(a);
+    sieve_of(mode)<<<grid, block, smem, s>>>(a);
 }
 
 namespace {

@@ -108,7 +108,10 @@ struct SumsArgs {
     i64 invw_count;
 };
 
-void launch_sieve(const SieveArgs& a, bool odd, int grid, int block, size_t smem, cudaStream_t s);
+// Sieve modes: every value, the odd values with u_dense on a 64-value word, and the odd values
+// of segments above 2 u_dense for any u_dense.
+enum { kSieveFull = 0, kSieveOdd = 1, kSieveOddAny = 2 };
+void launch_sieve(const SieveArgs& a, int mode, int grid, int block, size_t smem, cudaStream_t s);
 // Bucketed squares: the multiples m*p^2 in (vlo, vhi] of the primes p = primes[first..n)
 // (p^2 > S: at most one per segment), counted per segment, then written per segment
 // in the order of off = exclusive scan of the counts (cur: zeroed cursors); bucket
@@ -210,7 +213,7 @@ void init_piece_constants();
 int record_error(int code, const char* msg);
 // Opt the sieve kernel into the shared memory of every segment length and report how many
 // CTAs of `block` threads with `smem` bytes fit on one SM.
-void sieve_kernel_attrs(size_t smem, bool odd, int block, int* per_sm);
+void sieve_kernel_attrs(size_t smem, int mode, int block, int* per_sm);
 // Segments [a, b) of an odd-mode launch that may follow launches covering [0, a):
 // the largest b such that the halves of every value of [a, b) lie below segment a.
 i64 sieve_odd_range_end(i64 a, i64 nseg, i64 dense_segs, i64 u_dense, i64 u_total, int S);

@@ -246,7 +246,7 @@ int dr_measure_peaks(int device, dr_peaks *out);
  * caller passes the four table buffers it allocated itself.  The build's
  * scratch -- per-segment Mobius sums and their offsets, the sieving primes,
  * the periodic stencil, per-prime reciprocals and marking work items -- is one
- * fixed 796,848-byte __device__ array inside libdrb200.so, which every GPU that
+ * fixed 655,072-byte __device__ array inside libdrb200.so, which every GPU that
  * loads the library holds until the process exits.
  *
  *   u_total in [1, DR_NOALLOC_MAX_U = 2^33]; larger sizes are rejected with
