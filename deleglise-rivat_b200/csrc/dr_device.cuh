@@ -334,7 +334,7 @@ constexpr u64 kTileMaxY = 1ull << 51;
 // block's first candidate (y W / (2 q^2) = kWinRun), and at the query's last window.  IEEE
 // operations only: host and device agree.
 constexpr int kTileWin = 98304;
-constexpr double kWinRun = 64.0;
+constexpr double kWinRun = 32.0;
 __host__ __device__ inline u64 tile_windows(u64 X, u64 blk, u64 twin_max) {
     const double y = (double)X / (double)(96 * blk + 1);
     const double w = sqrt(y * (1.0 / (2.0 * kWinRun * kTileWin)));

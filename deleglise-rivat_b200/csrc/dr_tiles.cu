@@ -40,6 +40,12 @@ struct __align__(16) TileMember {
     int32_t pad;
 };
 
+// one 16-byte read (left to itself the compiler reads yd and sg separately)
+__device__ __forceinline__ TileMember member_of(const TileMember* p) {
+    const int4 v = *reinterpret_cast<const int4*>(p);
+    return TileMember{__hiloint2double(v.y, v.x), v.z, 0};
+}
+
 // One warp's state: the members of the group and, where a block reaches past the range of
 // some member, their ranges (S1: index range, S2: j range).
 struct TileWarp {
@@ -79,7 +85,7 @@ __device__ __forceinline__ int s1_lanes_n(const int16_t* dMm1, const TileWarp& W
     int s = 0;
 #pragma unroll 2
     for (int m = ma; m < mb; ++m) {
-        const TileMember E = W.e[m];
+        const TileMember E = member_of(&W.e[m]);
         int v[4];
         if (MASK) {
             const uint2 R = W.r[m];
@@ -161,7 +167,7 @@ struct TileAcc<true> {
 template <int KIND, bool MASK, bool WIDE>
 __device__ __forceinline__ i64 s2_tile(const TileWarp& W, const int32_t* sT, int32_t a12, const uint32_t* j,
                                        const double* r, const int32_t* mu, int ma, int mb, uint32_t pos,
-                                       uint32_t neg) {
+                                       uint32_t neg, bool exact) {
     typedef typename TileAcc<WIDE>::type A;
     A acc[4] = {0, 0, 0, 0};
     int32_t t[4] = {0, 0, 0, 0};
@@ -169,14 +175,16 @@ __device__ __forceinline__ i64 s2_tile(const TileWarp& W, const int32_t* sT, int
     double r12[4];
     if (KIND == 0) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {  // RN(1/(12 j)) to the last bit or so: one Newton step
-            const double q = r[c] * (1.0 / 12.0);
-            r12[c] = __fma_rn(q, __fma_rn(-12.0 * u32_double(j[c]), q, 1.0), q);
+        for (int c = 0; c < 4; ++c) r12[c] = r[c] * (1.0 / 12.0);
+        if (exact) {  // RN(1/(12 j)) to the last bit or so: one Newton step
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                r12[c] = __fma_rn(r12[c], __fma_rn(-12.0 * u32_double(j[c]), r12[c], 1.0), r12[c]);
         }
     }
-#pragma unroll 2
+#pragma unroll(MASK || KIND == 0 ? 1 : 2)
     for (int m = ma; m < mb; ++m) {
-        const TileMember E = W.e[m];
+        const TileMember E = member_of(&W.e[m]);
         uint2 R = make_uint2(0u, 0u);
         if (MASK) R = W.r[m];
 #pragma unroll
@@ -199,24 +207,30 @@ __device__ __forceinline__ i64 s2_tile(const TileWarp& W, const int32_t* sT, int
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
         const int32_t p = KIND >= 2 ? __popc(par[c] & pos) - __popc(par[c] & neg) : 0;
-        i64 v;
-        if (KIND == 1) v = (i64)acc[c];
-        else if (KIND == 2) v = ((i64)acc[c] + p) >> 1;  // an even sum
+        A v;  // every summand is at most its quotient: the sum fits A as the quotients' does
+        if (KIND == 1) v = acc[c];
+        else if (KIND == 2) v = (acc[c] + p) >> 1;  // an even sum
         else if (KIND == 3) v = p;
-        else if (KIND == 4) v = (i64)acc[c] + p;
-        else v = (i64)a12 * (i64)acc[c] + t[c];
-        s += (i64)mu[c] * v;
+        else if (KIND == 4) v = acc[c] + p;
+        else v = (A)a12 * acc[c] + t[c];
+        s += (i64)mu[c] * (i64)v;
     }
     return s;
 }
 
-// mu(j) and RN(1/j) of the two j of wheel position m, j[0] = 6m+1 and j[1] = 6m+5.  invw's
-// reciprocals are up to 3.5 ulp off (mu in the low bits): one Newton step brings them to
-// within 2^-53 (1 + 2^-40) of 1/j.
-__device__ __forceinline__ void wheel_pair(const SumsArgs& a, uint32_t m, double* r, int32_t* mu) {
-    const double2 iv = __ldg(a.invw + m);
-    r[0] = __fma_rn(iv.x, __fma_rn(-u32_double(6u * m + 1u), iv.x, 1.0), iv.x);
-    r[1] = __fma_rn(iv.y, __fma_rn(-u32_double(6u * m + 5u), iv.y, 1.0), iv.y);
+// mu(j) and 1/j of the two j of wheel position m, j[0] = 6m+1 and j[1] = 6m+5.  invw's
+// reciprocals are up to 3.5 ulp off (mu in the low bits), which leaves (y + 1/2) r between the
+// same two integers while y < 2^48 (2^48 * 7 * 2^-53 < 1/2, and r/12 adds two roundings:
+// 2^48 * 9 * 2^-53 < 1/2).  Above (`exact`), one Newton step brings them to within 2^-53
+// (1 + 2^-40) of 1/j.
+constexpr double kExactRcpY = 281474976710656.0;  // 2^48
+__device__ __forceinline__ void wheel_pair(const double2 iv, uint32_t m, double* r, int32_t* mu, bool exact) {
+    r[0] = iv.x;
+    r[1] = iv.y;
+    if (exact) {
+        r[0] = __fma_rn(iv.x, __fma_rn(-u32_double(6u * m + 1u), iv.x, 1.0), iv.x);
+        r[1] = __fma_rn(iv.y, __fma_rn(-u32_double(6u * m + 5u), iv.y, 1.0), iv.y);
+    }
     mu[0] = (int32_t)((uint32_t)__double2loint(iv.x) << 30) >> 30;
     mu[1] = (int32_t)((uint32_t)__double2loint(iv.y) << 30) >> 30;
 }
@@ -228,7 +242,7 @@ __device__ __noinline__ i64 s2_any(const SumsArgs& a, const TileWarp& W, const i
     for (uint32_t m = m0 + (uint32_t)lane; m < m0 + kTileM && m <= mmax; m += 32) {
         double r[2];
         int32_t mu[2];
-        wheel_pair(a, m, r, mu);
+        wheel_pair(__ldg(a.invw + m), m, r, mu, true);
         for (int h = 0; h < 2; ++h) {
             const uint32_t j = 6u * m + (h ? 5u : 1u);
             const double rj = h ? r[1] : r[0];
@@ -247,10 +261,10 @@ __device__ __noinline__ i64 s2_any(const SumsArgs& a, const TileWarp& W, const i
 template <int KIND>
 __device__ __forceinline__ i64 s2_block(const TileWarp& W, const int32_t* sT, int32_t a12, const uint32_t* j,
                                         const double* r, const int32_t* mu, int ma, int mb, uint32_t pos,
-                                        uint32_t neg, bool core, bool wide) {
-    if (wide) return s2_tile<KIND, true, true>(W, sT, a12, j, r, mu, ma, mb, pos, neg);
-    if (core) return s2_tile<KIND, false, false>(W, sT, a12, j, r, mu, ma, mb, pos, neg);
-    return s2_tile<KIND, true, false>(W, sT, a12, j, r, mu, ma, mb, pos, neg);
+                                        uint32_t neg, bool core, bool wide, bool exact) {
+    if (wide) return s2_tile<KIND, true, true>(W, sT, a12, j, r, mu, ma, mb, pos, neg, exact);
+    if (core) return s2_tile<KIND, false, false>(W, sT, a12, j, r, mu, ma, mb, pos, neg, exact);
+    return s2_tile<KIND, true, false>(W, sT, a12, j, r, mu, ma, mb, pos, neg, exact);
 }
 
 // kind of piece 1..12 (piece_kind of sums_kernel)
@@ -411,13 +425,14 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
                             s2 += (u64)s2_any(a, W, T, a12, m0, uhi, ma, mb, lane);
                             continue;
                         }
+                        const bool exact = !(y_hi < kExactRcpY);
                         uint32_t j[4];
                         double r[4];
                         int32_t mu[4];
 #pragma unroll
                         for (int p = 0; p < 2; ++p) {
                             const uint32_t m = m0 + 32u * p + (uint32_t)lane;
-                            wheel_pair(a, min(m, uhi), r + 2 * p, mu + 2 * p);
+                            wheel_pair(__ldg(a.invw + min(m, uhi)), min(m, uhi), r + 2 * p, mu + 2 * p, exact);
                             j[2 * p] = 6u * m + 1u;  // past uhi: outside every member's range
                             j[2 * p + 1] = 6u * m + 5u;
                         }
@@ -426,11 +441,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
                         const uint32_t pos = (rpos >> ma) << (32 - (mb - ma)), neg = (rneg >> ma) << (32 - (mb - ma));
                         i64 v;
                         switch (kind) {
-                        case 1: v = s2_block<1>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide); break;
-                        case 2: v = s2_block<2>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide); break;
-                        case 3: v = s2_block<3>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide); break;
-                        case 4: v = s2_block<4>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide); break;
-                        default: v = s2_block<0>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide); break;
+                        case 1: v = s2_block<1>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide, exact); break;
+                        case 2: v = s2_block<2>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide, exact); break;
+                        case 3: v = s2_block<3>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide, exact); break;
+                        case 4: v = s2_block<4>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide, exact); break;
+                        default: v = s2_block<0>(W, T, a12, j, r, mu, ma, mb, pos, neg, core, wide, exact); break;
                         }
                         s2 += (u64)v;
                     }

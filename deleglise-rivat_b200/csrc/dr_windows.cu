@@ -26,6 +26,9 @@ namespace drb {
 namespace {
 
 constexpr int kWinCta = 1024;
+// Union of index ranges below which the lanes take the members and the divisors come in turn
+// (with windows down to 32 divisors instead of 64: M(10^17) sums 100.8 -> 98.8 ms).
+constexpr uint32_t kNarrow = 48;
 
 struct __align__(16) WinMember {
     double yd;   // y + 1/2
@@ -57,7 +60,8 @@ __device__ __forceinline__ int win_block(uint32_t base, const WinMember* E, cons
     int s = 0;
 #pragma unroll 2
     for (int m = ma; m < mb; ++m) {
-        const WinMember M = E[m];
+        const int4 mv = *reinterpret_cast<const int4*>(E + m);  // one 16-byte read
+        const WinMember M{__hiloint2double(mv.y, mv.x), mv.z, 0};
         int v[4];
         if (MASK) {
             const uint2 g = R[m];
@@ -201,6 +205,26 @@ __global__ void __launch_bounds__(kWinCta, 1024 / kWinCta) windows_kernel(const 
                 res = __reduce_max_sync(0xffffffffu, member && cnt > 0 ? res : 0u);
                 const uint32_t tot = __reduce_add_sync(0xffffffffu, some ? (uint32_t)hi - lo + 1u : 0u);
                 const int sgn = ((dbits >> 2) & 1u) == ((dbits >> (5 + 3 * g)) & 1u) ? 1 : -1;
+                if (umax - umin < kNarrow) {
+                    // few divisors, all members at once: lanes on members, the divisors in turn
+                    double* rs = reinterpret_cast<double*>(R);
+                    int part = 0;
+                    for (uint32_t c = mine; 32u * c <= umax - umin; c += step) {
+                        const uint32_t i0 = umin + 32u * c;
+                        __syncwarp();
+                        rs[lane] = __ldg(a.rcp + tile_n(code, min(i0 + (uint32_t)lane, umax), res));
+                        __syncwarp();
+                        const int cnt = (int)min(32u, umax - i0 + 1u);
+#pragma unroll 4
+                        for (int t = 0; t < cnt; ++t) {
+                            const uint32_t i = i0 + (uint32_t)t;
+                            if (some && i >= lo && i <= (uint32_t)hi) part += win_M(base, floor_q(yd, rs[t]));
+                        }
+                    }
+                    acc += (i64)(sgn * part);
+                    __syncwarp();
+                    continue;
+                }
                 __syncwarp();
                 if (member) {
                     E[rank].sg = sgn;
