@@ -318,10 +318,11 @@ static_assert(sizeof(SlotDesc) == 96, "SlotDesc is six 16-byte words");
 constexpr u64 kSlotS1Only = 1ull << 15;
 
 // Tile groups (dr_tiles.cu): the evaluations e of a 32-candidate block of a query that
-// agree in kind and strides are summed together, one divisor range for all of them.
-// kSlotTile marks the slots that take part; the group's first slot (its leader) holds the
-// group's work, counted in units of kTileN divisors of an S1 segment or kTileM wheel
-// positions of an S2 piece over the union of the members' ranges.
+// agree in kind and strides are summed together, one divisor range for all of them (nearly
+// always one group to a block; a block that straddles a range boundary holds a few).
+// kSlotTile marks the slots that take part.  Work is counted per (block, e) in units of
+// kTileN divisors of an S1 segment or kTileM wheel positions of an S2 piece over the union of
+// the members' ranges.
 constexpr u64 kSlotTile = 1ull << 16;
 constexpr uint32_t kTileN = 128;
 constexpr uint32_t kTileM = 64;
@@ -340,6 +341,14 @@ __host__ __device__ inline u64 tile_windows(u64 X, u64 blk, u64 twin_max) {
     const double w = sqrt(y * (1.0 / (2.0 * kWinRun * kTileWin)));
     return w < (double)twin_max ? (u64)w : twin_max;
 }
+
+// The units of a (block, e) of one group as the tile kernel finds them: segment g takes the
+// units [end[g - 1], end[g]) and the index range [lo[g], hi[g]].
+struct __align__(16) TileGroup {
+    uint32_t end[kS1Seg + 8], lo[kS1Seg + 8], hi[kS1Seg + 8];
+    uint32_t single;  // one group (else the tile kernel works them out again)
+    uint32_t pad[3];
+};
 
 // A tile group as the window kernel (dr_windows.cu) reads it.
 struct __align__(16) WinGroup {

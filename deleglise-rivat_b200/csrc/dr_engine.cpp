@@ -90,6 +90,7 @@ struct dr_ctx {
     // query buffers
     DevBuf queries, ops, prefix, scan_tmp, misc, inv, invw, wdesc, witems, slots;
     DevBuf acc;             // results: 3 sums and kCountsPerQuery counters per query, then 4 words of work queues
+    DevBuf tgroups;         // tile kernel: units of each (block, e)
     DevBuf groups, titems;  // window kernel: tile groups; work items and tasks
     // table state
     bool table_valid = false;
@@ -195,7 +196,7 @@ bool release_scratch(dr_ctx* c) {
     DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->consts, &c->queries,
                       &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->misc, &c->inv, &c->invw, &c->wdesc, &c->witems,
                       &c->slots, &c->sq_cnt, &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp, &c->dplanes, &c->bplanes,
-                      &c->bckpt, &c->groups, &c->titems};
+                      &c->bckpt, &c->tgroups, &c->groups, &c->titems};
     bool any = false;
     for (DevBuf* b : bufs) {
         any = any || b->p;
@@ -1089,10 +1090,14 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     u64* const acc = (u64*)c->acc.p;
     i64* const counts = (i64*)(acc + 3 * nq);
     u64* const ticket = acc + (size_t)nq * (3 + kCountsPerQuery);
-    if ((rc = ensure(c, c->ops, (size_t)std::max<u64>(slots, 1) * 8))) return rc;
-    if ((rc = ensure(c, c->prefix, (size_t)(slots + 1) * 8))) return rc;
+    // ops per slot for the sums kernel (the windowed S1, the bands, what the tile kernel
+    // leaves), per (block, e) for the tile kernel
+    const u64 n_ops = !witems.empty() || sp || rest ? std::max(slots, 2 * blocks) : 2 * blocks;
+    if ((rc = ensure(c, c->ops, (size_t)std::max<u64>(n_ops, 1) * 8))) return rc;
+    if ((rc = ensure(c, c->prefix, (size_t)(n_ops + 1) * 8))) return rc;
+    if (witems.empty() && (rc = ensure(c, c->tgroups, (size_t)std::max<u64>(2 * blocks, 1) * sizeof(TileGroup)))) return rc;
     if ((rc = ensure(c, c->slots, (size_t)std::max<u64>(slots, 1) * sizeof(SlotDesc)))) return rc;
-    if ((rc = ensure(c, c->scan_tmp, scan_u64_tmp_elems(slots) * 8))) return rc;
+    if ((rc = ensure(c, c->scan_tmp, scan_u64_tmp_elems(n_ops) * 8))) return rc;
     if (!witems.empty()) {
         if ((rc = ensure(c, c->wdesc, (size_t)std::max<u64>(slots, 1) * sizeof(S1WinDesc)))) return rc;
         if ((rc = ensure(c, c->witems, witems.size() * sizeof(S1WinItem)))) return rc;
@@ -1166,9 +1171,11 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         // a streamed table: this pass takes the S1 lookups with q <= u_res, the bands the rest
         launch_plan((const QueryDev*)c->queries.p, qn, T, blocks, (u64*)c->ops.p, acc, counts,
                     sw ? (S1WinDesc*)c->wdesc.p : nullptr, (SlotDesc*)c->slots.p, c->sm_count, c->stream, band,
-                    tiles ? kPlanTiles : kPlanSlots, windows ? (WinGroup*)c->groups.p : nullptr);
-        launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
-                        scan_u64_tmp_elems(slots), c->stream);
+                    tiles ? kPlanTiles : kPlanSlots, tiles ? (TileGroup*)c->tgroups.p : nullptr,
+                    windows ? (WinGroup*)c->groups.p : nullptr);
+        const u64 n_scan = tiles ? 2 * blocks : slots;
+        launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, n_scan, (u64*)c->scan_tmp.p,
+                        scan_u64_tmp_elems(n_scan), c->stream);
         launches += 5;
     }
     CU(cudaGetLastError());
@@ -1194,6 +1201,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         sa.T = T;
         sa.n_slots = slots;
         sa.n_blocks = blocks;
+        sa.tgroups = tiles ? (const TileGroup*)c->tgroups.p : nullptr;
         sa.prefix = (const u64*)c->prefix.p;
         sa.slots = (const SlotDesc*)c->slots.p;
         sa.ticket = ticket;
@@ -1451,7 +1459,7 @@ int dr_ctx_destroy(dr_ctx* c) {
     DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->consts, &c->stencil,
                       &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->misc, &c->inv, &c->invw, &c->wdesc,
                       &c->witems, &c->slots, &c->sq_cnt, &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp,
-                      &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->groups, &c->titems};
+                      &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->tgroups, &c->groups, &c->titems};
     for (DevBuf* b : bufs) release(c, *b);
     drop_graphs(c);
     if (c->pinned) cudaFreeHost(c->pinned);

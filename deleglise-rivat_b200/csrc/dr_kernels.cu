@@ -1030,13 +1030,13 @@ __device__ __forceinline__ int query_of_block(const QueryDev* q, int nq, u64 b) 
 // streamed table, band.s1_only, counts only its S1 lookups and adds no constant part: those
 // belong to the resident pass).  mode:
 //   kPlanSlots  ops[s] = the slot's lookups and positions, for sums_kernel
-//   kPlanTiles  ops of a tile group's leader = its units, for the tile kernel; 0 elsewhere
+//   kPlanTiles  ops[w] = the units of (block, e) w = 2*block + e, for the tile kernel
 //   kPlanRest   ops[s] as kPlanSlots where the slot is not tile-eligible, else 0; the
 //               constants and counters were the kPlanTiles pass's
 __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const TableView T, u64 n_blocks,
                             u64* __restrict__ ops, u64* __restrict__ acc, i64* __restrict__ counts,
                             S1WinDesc* __restrict__ wdesc, SlotDesc* __restrict__ slots, const S1Band band,
-                            const int mode, WinGroup* __restrict__ groups) {
+                            const int mode, TileGroup* __restrict__ tgroups, WinGroup* __restrict__ groups) {
     const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
     const int lane = threadIdx.x & 31;
     for (u64 w = (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < 2 * n_blocks; w += warps) {
@@ -1149,13 +1149,12 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
                 }
                 if (lane == 0) groups[w] = G;
             }
-            u64 units = 0;
-            while (left) {
-                const int lead = __ffs(left) - 1;
-                const u64 lead_sig = __shfl_sync(0xffffffffu, sig, lead);
+            uint32_t units = 0, rlo = 1, rhi = 0, rend = 0;
+            int ngroups = 0;
+            for (; left; ++ngroups) {
+                const u64 lead_sig = __shfl_sync(0xffffffffu, sig, __ffs(left) - 1);
                 const bool member = tile && sig == lead_sig;
                 left &= ~__ballot_sync(0xffffffffu, member);
-                uint32_t sum = 0;
 #pragma unroll
                 for (int g = 0; g < kS1Seg + 8; ++g) {
                     uint32_t lo = 1, hi = 0, res;
@@ -1163,11 +1162,19 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
                     if (member) tile_range(t, g, &lo, &hi, &res, &jr);
                     const uint32_t ulo = __reduce_min_sync(0xffffffffu, lo <= hi ? lo : 0xffffffffu);
                     const uint32_t uhi = __reduce_max_sync(0xffffffffu, lo <= hi ? hi : 0u);
-                    sum += tile_units(g, ulo, uhi);
+                    units += tile_units(g, ulo, uhi);
+                    if (lane == g) rlo = ulo, rhi = uhi, rend = units;
                 }
-                if (lane == lead) units = sum;
             }
-            if (valid) ops[s] = units;
+            if (lane < kS1Seg + 8) {
+                tgroups[w].end[lane] = rend;
+                tgroups[w].lo[lane] = rlo;
+                tgroups[w].hi[lane] = rhi;
+            }
+            if (lane == 0) {
+                tgroups[w].single = ngroups == 1 ? 1u : 0u;
+                ops[w] = units;
+            }
         }
         if (mode == kPlanRest) continue;
 #pragma unroll
@@ -1184,10 +1191,10 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
 
 void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc, i64* counts,
                  S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s, const S1Band& band, int mode,
-                 WinGroup* groups) {
+                 TileGroup* tgroups, WinGroup* groups) {
     if (n_blocks == 0) return;
     const int grid = (int)std::min<u64>((2 * n_blocks + 3) / 4, (u64)sm_count * 16);
-    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode, groups);
+    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode, tgroups, groups);
 }
 
 // Direct answers for queries with X <= table u_total (get_M, :1465-1467).

@@ -98,6 +98,7 @@ struct SumsArgs {
     u64 n_slots;
     u64 n_blocks;       // 32-candidate blocks of all queries
     const u64* prefix;  // [n_slots + 1] exclusive op prefix
+    const TileGroup* tgroups;  // [2 * n_blocks], tile kernel only (prefix then runs over these)
     const SlotDesc* slots;  // [n_slots] each slot's evaluation, written by plan_kernel
     u64* ticket;        // [0]: work-queue counter, [1]: error flag; zeroed before launch
     u64* acc;           // [3 * nq]: C, S1, S2
@@ -168,7 +169,7 @@ constexpr int kBandInThread = 64;
 enum { kPlanSlots = 0, kPlanTiles = 1, kPlanRest = 2 };
 void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc,
                  i64* counts, S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s,
-                 const S1Band& band, int mode, WinGroup* groups = nullptr);
+                 const S1Band& band, int mode, TileGroup* tgroups = nullptr, WinGroup* groups = nullptr);
 // Windowed S1 (window length win: a power of two, 2^12 .. 2^16).
 void launch_s1win(const S1WinArgs& a, u64 win, int sm_count, cudaStream_t s);
 void launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t tmp_elems, cudaStream_t s);

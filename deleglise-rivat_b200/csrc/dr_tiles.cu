@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
     TileWarp& W = sw[threadIdx.x >> 5];
     const int16_t* dMm1 = a.T.dM - 1;  // dMm1[q] = M(q)
     const double dense_q = (double)min(a.T.u_dense, (i64)0xFFFFFFFEll);
-    const u64 total = a.prefix[a.n_slots];
+    const u64 n_groups = 2 * a.n_blocks, total = a.prefix[n_groups];
     // Units per ticket: neighbouring units of a group share its set-up and table lines in L1,
     // so up to 64 (32: 2% more at M(10^16), 4% at the 256-query batch), but 16 tickets per warp
     // so that the last ones do not wait for one long one (8 tickets of up to 128: 2.0 -> 2.5 ms
@@ -299,14 +299,18 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
         if (o >= total) break;
         const u64 o_end = min(o + per, total);
         while (o < o_end) {
-            const u64 s = warp_upper_slot(a.prefix, a.n_slots, o, lane);
-            const u64 sbase = a.prefix[s], send = a.prefix[s + 1];
+            const u64 w = warp_upper_slot(a.prefix, n_groups, o, lane);
+            const u64 sbase = a.prefix[w], send = a.prefix[w + 1];
+            const TileGroup* rec = a.tgroups + w;
+            const bool single = __ldg(&rec->single) != 0;
+            uint32_t rend = 0, rlo = 1, rhi = 0;
+            if (lane < kS1Seg + 8) rend = __ldg(rec->end + lane), rlo = __ldg(rec->lo + lane), rhi = __ldg(rec->hi + lane);
             int qi = 0;
             if (a.nq > 1) {
                 int lo = 0, hi = a.nq - 1;
                 while (lo < hi) {
                     const int mid = (lo + hi + 1) >> 1;
-                    if (a.queries[mid].slot_base <= s) lo = mid;
+                    if (a.queries[mid].blk_base <= w >> 1) lo = mid;
                     else hi = mid - 1;
                 }
                 qi = lo;
@@ -322,33 +326,48 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
                 s1 = s2 = 0;
                 cur_q = qi;
             }
-            // the group led by slot s: its members, one per lane
+            // the block's evaluations, one per lane
             const u64 slot_base = a.queries[qi].slot_base;
-            const u64 nc = (u64)a.queries[qi].nc;
-            const u64 local = s - slot_base;
-            const u64 cand = local >> 1;
-            const u64 c = (cand & ~31ull) + (u64)lane;
-            const SlotDesc* mine = a.slots + (slot_base + 2 * c + (local & 1));
-            const u64 bits = c < nc ? mine->bits : 0ull;
-            const u64 sig = __shfl_sync(0xffffffffu, bits & (kSlotTile | kTileSig), (int)(cand & 31u));
-            const bool member = (sig & kSlotTile) && (bits & (kSlotTile | kTileSig)) == sig;
+            const u64 c = 32 * ((w >> 1) - a.queries[qi].blk_base) + (u64)lane;
+            const SlotDesc* mine = a.slots + (slot_base + 2 * c + (w & 1));
+            const bool there = c < (u64)a.queries[qi].nc;
+            const u64 bits = there ? mine->bits : 0ull;
+            const double y_own = there ? (double)(i64)mine->y + 0.5 : 0.0;
+            unsigned left = __ballot_sync(0xffffffffu, (bits & kSlotTile) != 0);
+            const u64 u0 = o - sbase, u1 = min(o_end, send) - sbase;  // this ticket's units
+            const uint32_t rstart = __shfl_up_sync(0xffffffffu, rend, 1);
+            const unsigned visit = __ballot_sync(0xffffffffu, lane < kS1Seg + 8 && rend > u0 &&
+                                                                  (lane == 0 ? 0u : rstart) < u1);
+            u64 useg = 0;
+            while (left && useg < u1) {
+            const u64 sig = __shfl_sync(0xffffffffu, bits & (kSlotTile | kTileSig), __ffs(left) - 1);
+            const bool member = (bits & (kSlotTile | kTileSig)) == sig;
             const unsigned mm = __ballot_sync(0xffffffffu, member);
+            left &= ~mm;
             const int rank = __popc(mm & ((1u << lane) - 1u));
-            const double yd = member ? (double)(i64)mine->y + 0.5 : 0.0;
+            const double yd = member ? y_own : 0.0;
             const uint32_t kbits = (uint32_t)sig;
             const int piece0 = (kbits & 3u) == EVAL_SINGLE ? 9 : 1;
-            const u64 u0 = o - sbase, u1 = min(o_end, send) - sbase;  // this ticket's units of the group
-            u64 useg = 0;
-            for (int g = 0; g < kS1Seg + 8 && useg < u1 && mm; ++g) {
+            for (unsigned gm = single ? visit : (1u << (kS1Seg + 8)) - 1u; gm; gm &= gm - 1u) {
+                const int g = __ffs(gm) - 1;
                 uint32_t lo = 1, hi = 0, res = 0;
                 uint2 jr = make_uint2(1u, 0u);
                 if (member) tile_range(*mine, g, &lo, &hi, &res, &jr);
                 const bool some = lo <= hi;
-                const uint32_t ulo = __reduce_min_sync(0xffffffffu, some ? lo : 0xffffffffu);
-                const uint32_t uhi = __reduce_max_sync(0xffffffffu, some ? hi : 0u);
-                const uint32_t units = tile_units(g, ulo, uhi);
-                const u64 ub = useg;
-                useg += units;
+                uint32_t ulo, uhi;
+                u64 ub;
+                if (single) {
+                    ulo = __shfl_sync(0xffffffffu, rlo, g);
+                    uhi = __shfl_sync(0xffffffffu, rhi, g);
+                    useg = __shfl_sync(0xffffffffu, rend, g);
+                    const uint32_t start = __shfl_sync(0xffffffffu, rstart, g);
+                    ub = g ? start : 0u;
+                } else {
+                    ulo = __reduce_min_sync(0xffffffffu, some ? lo : 0xffffffffu);
+                    uhi = __reduce_max_sync(0xffffffffu, some ? hi : 0u);
+                    ub = useg;
+                    useg += tile_units(g, ulo, uhi);
+                }
                 const u64 a0 = max(u0, ub), a1 = min(u1, useg);
                 if (a0 >= a1) continue;
                 const bool plus = !(bits & 4u);
@@ -450,6 +469,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, 2) tiles_kernel(const SumsArg
                         s2 += (u64)v;
                     }
                 }
+            }
             }
             if (useg < u1) {
                 // planning and this kernel disagree on the group's units: flag it and go on
