@@ -355,8 +355,8 @@ class Engine:
         """(M[first:first+count], mu[...]) as numpy arrays (get_M / get_mu)."""
         import numpy as np
 
-        M = np.zeros(count, dtype=np.int32)
-        mu = np.zeros(count, dtype=np.int8)
+        M = np.empty(count, dtype=np.int32)
+        mu = np.empty(count, dtype=np.int8)
         _check(lib().dr_table_read(self._ctx, int(first), int(count),
                                    M.ctypes.data_as(ctypes.POINTER(ctypes.c_int32)),
                                    mu.ctypes.data_as(ctypes.POINTER(ctypes.c_int8))))
@@ -365,7 +365,7 @@ class Engine:
     def table_read_wheel(self, first: int, count: int):
         import numpy as np
 
-        mu = np.zeros(count, dtype=np.int8)
+        mu = np.empty(count, dtype=np.int8)
         _check(lib().dr_table_read_wheel(self._ctx, int(first), int(count),
                                          mu.ctypes.data_as(ctypes.POINTER(ctypes.c_int8))))
         return mu
