@@ -84,6 +84,7 @@ struct dr_ctx {
     // streamed table (dr_ctx_set_resident_limit): above u_resident the compressed tier
     // is built and consumed band by band in these two buffers, never held whole
     DevBuf bplanes, bckpt;
+    DevBuf kplanes;  // plane words of the bands below u_total/2, where the bands above find their halves
     int64_t u_resident = 0, band_values = 0;
     std::vector<cudaEvent_t> bev;  // band timing: start, then per band after its build and after its sums
     int64_t last_bands = 0;        // bands the enqueued call streams
@@ -196,7 +197,7 @@ bool release_scratch(dr_ctx* c) {
     DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->consts, &c->queries,
                       &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->misc, &c->inv, &c->invw, &c->wdesc, &c->witems,
                       &c->slots, &c->sq_cnt, &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp, &c->dplanes, &c->bplanes,
-                      &c->bckpt, &c->tgroups, &c->groups, &c->titems};
+                      &c->bckpt, &c->kplanes, &c->tgroups, &c->groups, &c->titems};
     bool any = false;
     for (DevBuf* b : bufs) {
         any = any || b->p;
@@ -854,16 +855,38 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
     }
     CU(cudaEventRecord(c->bev[0], c->stream));
     c->last_bands = sp.nbands;
+    // The bands below u_total/2 keep their plane words where there is room (every other buffer
+    // of the call is in place), so that the bands above find all their halves there or in the
+    // resident table and run in odd mode too: M(10^16) with 6e9 of 2.27e10 values resident
+    // 54.2 -> 43.4 ms.
+    const int64_t w_res = (sp.nseg_res - sp.dense_segs) * (S / 64);
+    int64_t kept = 0;  // bands [0, kept)
+    if (odd_ok) {
+        while (kept < sp.nbands) {
+            int64_t vlo, vhi;
+            band_values_of(sp, kept, &vlo, &vhi);
+            if (vlo >= sp.u_total / 2) break;
+            ++kept;
+        }
+        if (kept == sp.nbands || ensure(c, c->kplanes, (size_t)kept * (size_t)sp.band_segs * (size_t)(S / 64) * 16)) kept = 0;
+        if (kept) {
+            ao.hsplit = w_res;
+            ao.hplanes2 = (const ulonglong2*)c->kplanes.p - w_res;
+        }
+    }
     for (int64_t b = 0; b < sp.nbands; ++b) {
         const int64_t c0 = band_first_seg(sp, b), c1 = std::min(sp.nseg, c0 + sp.band_segs);
         int64_t vlo, vhi;
         band_values_of(sp, b, &vlo, &vhi);
         const int64_t cword0 = (c0 - sp.dense_segs) * (S / 64);
-        const bool odd = band_odd(sp, vlo, vhi);
+        const bool odd = band_odd(sp, vlo, vhi) ||
+                         (kept && vlo >= 2 * sp.u_dense && vhi + 2 * (int64_t)S <= 2 * vlo);
+        ulonglong2* const planes = b < kept ? (ulonglong2*)c->kplanes.p + (cword0 - w_res) : (ulonglong2*)c->bplanes.p;
         SieveArgs& m = odd ? ao : a;
         m.seg_begin = c0;
         m.seg_end = c1;
         m.cword0 = cword0;
+        m.planes = planes;
         m.sq_off = nullptr;
         m.sq_pos = nullptr;
         m.sq_seg0 = c0;
@@ -892,7 +915,7 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
         CU(cudaGetLastError());
         CU(cudaEventRecord(c->bev[(size_t)(2 * b + 1)], c->stream));
         SumsArgs sa = base;
-        sa.T.planes = (const ulonglong2*)c->bplanes.p;
+        sa.T.planes = planes;
         sa.T.ckpt = (const int32_t*)c->bckpt.p;
         sa.T.cbase = cword0;
         CU(cudaMemsetAsync(sa.ticket, 0, 8, c->stream));  // the work-queue counter (not the error flag)
@@ -1459,7 +1482,7 @@ int dr_ctx_destroy(dr_ctx* c) {
     DevBuf* bufs[] = {&c->dM, &c->planes, &c->ckpt, &c->wheel, &c->seg_sum, &c->seg_off, &c->consts, &c->stencil,
                       &c->queries, &c->ops, &c->prefix, &c->scan_tmp, &c->acc, &c->misc, &c->inv, &c->invw, &c->wdesc,
                       &c->witems, &c->slots, &c->sq_cnt, &c->sq_off, &c->sq_cur, &c->sq_pos, &c->sq_tmp,
-                      &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->tgroups, &c->groups, &c->titems};
+                      &c->stencil_odd, &c->dplanes, &c->bplanes, &c->bckpt, &c->kplanes, &c->tgroups, &c->groups, &c->titems};
     for (DevBuf* b : bufs) release(c, *b);
     drop_graphs(c);
     if (c->pinned) cudaFreeHost(c->pinned);

@@ -59,6 +59,8 @@ struct SieveArgs {
     const ulonglong2* hplanes; // the compressed tier's plane words from word 0, where odd mode
                                // reads the halves (planes itself, or the resident table's
                                // planes for a streamed band whose halves are resident)
+    i64 hsplit = INT64_MAX;    // from this word on, word w is hplanes2[w] (the kept planes of
+    const ulonglong2* hplanes2 = nullptr;  // earlier bands)
     uint4* wheel;
     int32_t* seg_sum;
 };

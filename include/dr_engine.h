@@ -107,8 +107,9 @@ int dr_ctx_set_hbm_budget(dr_ctx *ctx, uint64_t bytes);
  * segment of the compressed tier, at least one segment above u_dense) in memory; the
  * compressed tier above is sieved band by band, band_values values at a time (0: as
  * many as the resident compressed tier holds), and after each band the S1 lookups
- * whose quotient falls in it are summed.  M(X) and the C/S1/S2 checksums are those
- * of the whole table.  Needs X > u_total and mu_limit <= u_res; batches never
+ * whose quotient falls in it are summed.  Where the budget has room the plane words
+ * of the bands below u_total/2 (0.25 bytes a value) are kept, which halves the work of
+ * the bands above.  M(X) and the C/S1/S2 checksums are those of the whole table.  Needs X > u_total and mu_limit <= u_res; batches never
  * stream.  u_resident = 0 (the default) holds every table whole.  The bands'
  * build and lookups count in dr_stats.sums_ms (split out in band_table_ms and
  * band_sums_ms). */
@@ -217,7 +218,9 @@ int64_t dr_debug_sieve_plan(int64_t u_total, int64_t u_dense, int32_t segment_lo
 /* The bands a streamed table (dr_ctx_set_resident_limit) of these limits would use --
  * test support, no counterpart in the reference: *u_res = the resident part's end
  * (u_total when nothing streams), then per band {vlo, vhi, odd}: its values (vlo, vhi]
- * and whether it is sieved in odd mode.  Writes at most cap triples; returns the band
+ * and whether it is sieved in odd mode by the resident table alone (a call also keeps
+ * the plane words of the bands below u_total/2 where its memory allows, and then runs
+ * the bands above in odd mode too).  Writes at most cap triples; returns the band
  * count (0: nothing streams) or a negative DR_ERR_* code.  Needs no GPU. */
 int64_t dr_debug_stream_plan(int64_t u_total, int64_t u_dense, int32_t segment_log2, int64_t u_resident,
                              int64_t band_values, int64_t *u_res, int64_t *out, int64_t cap);
