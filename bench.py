@@ -2,7 +2,7 @@
 """bench.py -- exact M(10^16) on B200 (seconds per M(X)) plus batched M(X)/s.
 
 One "step" is one complete M(10^16) through the engine: segmented Mobius sieve,
-dense + compressed Mertens tables, term planning, persistent S1/S2 kernel and
+dense + compressed Mertens tables, term planning, persistent S1/S2 kernels and
 the reduction -- nothing cached between steps (the ~9 GB of tables and
 reciprocals are rebuilt every step, far larger than the 126 MB L2).
 
@@ -254,20 +254,20 @@ def sieve_marks(u_total, u_dense, sm_count, S=1 << 17):
 
 # Warp instructions per unit of work, from ncu smsp__inst_executed.sum of one launch
 # divided by that launch's work:
-#   sums_kernel at M(10^15) (B200 policy): 7.05e9 instructions for 5.98e9 S1 lookups +
-#     2.40e9 S2 wheel positions; the S2 positions at 1.50 each (timing-only capture that
-#     keeps only the S2 part), the rest, 0.58 per lookup, to S1;
+#   S1/S2 phase at M(10^16) (B200 policy), tile and window kernels: the S2 positions
+#     (timing-only build that keeps only them) 4.95e9 instructions for 1.12e10 positions,
+#     the S1 lookups (window kernel, and the tile kernel without S2) 7.05e9 for 2.79e10;
 #   sieve_kernel, odd mode, on the M(10^15) table: 5.63e7 instructions for 1.01e8 values.
-SUMS_INST_PER_S1 = 0.58
-SUMS_INST_PER_S2 = 1.50
+SUMS_INST_PER_S1 = 0.253
+SUMS_INST_PER_S2 = 0.442
 SIEVE_INST_PER_VALUE = 0.556
-# DRAM bytes per op of sums_kernel (dram__bytes_read.sum + dram__bytes_write.sum of one
-# launch over its S1 lookups + S2 positions) at M(10^15): 10.71 GB / 8.38e9 ops.
-SUMS_DRAM_PER_OP = 1.28
+# DRAM bytes per op of the S1/S2 phase (dram__bytes_read.sum + dram__bytes_write.sum of the
+# tile and the window kernel over S1 lookups + S2 positions) at M(10^15): 8.25 GB / 7.80e9 ops.
+SUMS_DRAM_PER_OP = 1.06
 
 
 def sums_roofline(st, sums_ms, peak, peak_kind, issue_peak, f_mhz):
-    """S1/S2 phase (sums_kernel) against HBM on the algorithmic bytes -- 2 B per
+    """S1/S2 phase (tile and window kernels) against HBM on the algorithmic bytes -- 2 B per
     dense-tier S1 lookup, 20 B per compressed-tier lookup (16 B plane pair + 4 B
     checkpoint), 1 B of Mobius value per S2 candidate j (two per wheel position) --
     and against its binding unit, instruction issue."""
@@ -276,17 +276,17 @@ def sums_roofline(st, sums_ms, peak, peak_kind, issue_peak, f_mhz):
     alg = 2.0 * dense + 20.0 * st.s1_comp_ops + 2.0 * st.s2_ops
     inst = SUMS_INST_PER_S1 * st.s1_ops + SUMS_INST_PER_S2 * st.s2_ops
     return {
-        "bound": "hbm", "kernel": "sums_kernel (S1/S2 phase)", "achieved": alg / t / 1e9, "peak": peak,
+        "bound": "hbm", "kernel": "tiles_kernel + windows_kernel (S1/S2 phase)", "achieved": alg / t / 1e9, "peak": peak,
         "unit": "GB/s", "frac": alg / t / 1e9 / peak, "peak_kind": peak_kind,
         "traffic": SUMS_DRAM_PER_OP * (st.s1_ops + st.s2_ops),
-        "traffic_basis": "ncu DRAM bytes per op of one sums_kernel launch at M(10^15), times this call's op count",
+        "traffic_basis": "ncu DRAM bytes per op of the phase's kernels at M(10^15), times this call's op count",
         "alg_bytes": alg,
         "ops": {"s1_lookups": st.s1_ops, "s1_compressed": st.s1_comp_ops, "s2_positions": st.s2_ops},
         "ops_per_s": (st.s1_ops + st.s2_ops) / t,
         "issue": {"bound": "instruction issue (binding)", "warp_inst": inst, "achieved": inst / t,
                   "peak": issue_peak, "unit": "warp instructions/s", "frac": inst / t / issue_peak,
                   "basis": f"{SUMS_INST_PER_S1} warp instructions per S1 lookup + {SUMS_INST_PER_S2} per S2 "
-                           f"position (ncu at M(10^15)); peak = SMs x 4 x {f_mhz:.0f} MHz"},
+                           f"position (ncu at M(10^16)); peak = SMs x 4 x {f_mhz:.0f} MHz"},
     }
 
 
