@@ -338,9 +338,12 @@ __device__ __forceinline__ void mark_item(uint32_t* buf32, const uint4 I, const 
 
 // ---------------------------------------------------------------------------
 // Segmented byte-log Mobius sieve + table outputs (ODD: odd values only).
+// At most 48 registers (no spills): 1024 threads of them leave room for the side stream's
+// scan and fix-up CTAs on the same SM.  The compiler's own choice, 60, does not: a table of
+// 10^9 values 0.92 -> 1.00 ms, 2.3*10^10 19.7 -> 20.8; 40 registers 0.97 and 20.9.
 // ---------------------------------------------------------------------------
 template <int MODE>
-__global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
+__global__ void __maxnreg__(48) sieve_kernel(const SieveArgs a) {
     constexpr bool ODD = MODE != kSieveFull, ANY = MODE == kSieveOddAny;
     extern __shared__ __align__(16) unsigned char smem[];
     uint8_t* buf = smem;
@@ -486,18 +489,23 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
                 atomicOr(&buf32[j >> 2], 0x80u << ((j & 3) * 8));
             }
         }
-        //    Offsets low mod p: on the 32-bit quotient route (qest/qfix) while
-        //    p <= low and low/p < 2^31, else from the 64-bit reciprocal.  Round k
+        //    First hits: with v = low, or in odd mode the index (low - 1)/2 of the first odd
+        //    value among the odd numbers -- there the odd multiples of p are the indices
+        //    congruent to (p - 1)/2 -- v mod p from floor(v/p), one FMA rounded down
+        //    (v < 2^51: exact, see dr_tiles.cu; only its low word is needed).  Against the
+        //    two-step 32-bit quotient with a 64-bit route beside it: 10^11 values 103.8 ->
+        //    96.7 ms, 2.3*10^10 20.3 -> 19.7, 2*10^9 as before.  Round k
         //    gives thread t the prime T*k + t (k even) or T*k + T-1-t (k odd): the
         //    small primes of each round (the most hits) alternate between the
         //    first and the last warps, which evens out the warps' marking before
         //    the barrier.
-        const double lowd = __ull2double_rn((u64)low);
+        const i64 v = ODD ? (low - 1) >> 1 : low;
+        const double vd = (double)v + 0.5;
         uint32_t p_n = 0;
         double rc_n = 0.0;
         if (a.tierB_first + tid < a.n_primes) {
             p_n = __ldg(a.primes + a.tierB_first + tid);
-            if (a.prcp) rc_n = __ldg(a.prcp + a.tierB_first + tid);
+            rc_n = __ldg(a.prcp + a.tierB_first + tid);
         }
         for (int k = 0, i = a.tierB_first + tid; i < a.n_primes; ++k) {
             const uint32_t p = p_n;  // loaded one iteration ahead
@@ -505,17 +513,18 @@ __global__ void __launch_bounds__(1024) sieve_kernel(const SieveArgs a) {
             const int inext = a.tierB_first + T * (k + 1) + ((k & 1) ? tid : T - 1 - tid);
             if (inext < a.n_primes) {
                 p_n = __ldg(a.primes + inext);
-                if (a.prcp) rc_n = __ldg(a.prcp + inext);
+                rc_n = __ldg(a.prcp + inext);
             }
             const uint32_t w = (32u - __clz(p - 1)) | 1u;
-            uint32_t r;
-            if (a.prcp && (u64)low >= p && ((u64)low >> 31) < p)
-                r = (uint32_t)low - qfix(qest(lowd, rc), (uint32_t)low, p) * p;
-            else
-                r = (uint32_t)umod_inv((u64)low, p, a.pinv[i]);
-            uint32_t d = r ? p - r : 0;
-            if (ODD && (d & 1u)) d += p;
-            mark_prime(buf32, ODD ? d >> 1 : d, p, w, (uint32_t)nb);
+            const uint32_t r = (uint32_t)v - floor_q(vd, rc) * p;  // v mod p
+            uint32_t j;
+            if (ODD) {
+                const uint32_t h = p >> 1;
+                j = h - r + (r > h ? p : 0u);
+            } else {
+                j = r ? p - r : 0u;
+            }
+            mark_prime(buf32, j, p, w, (uint32_t)nb);
             i = inext;
         }
         __syncthreads();

@@ -42,7 +42,7 @@ struct SieveArgs {
     const uint32_t* primes;
     const u64* pinv;           // floor((2^64-1)/p) per prime: segment offsets without division
     const u64* sqinv;          // floor((2^64-1)/p^2) per prime
-    const double* prcp;        // RN(1/p) per prime (32-bit offset route; NULL: umod_inv only)
+    const double* prcp;        // RN(1/p) per prime: first hits by one FMA
     int sqC_first;             // first prime whose square is bucketed (p^2 > S); n_primes: none
     const u64* sq_off;         // bucketed square hits of each segment from sq_seg0 on (NULL: no bucket)
     i64 sq_seg0;               // segment of sq_off[0] (0, or a streamed band's first segment)
