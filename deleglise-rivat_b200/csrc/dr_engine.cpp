@@ -858,7 +858,8 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
     // The bands below u_total/2 keep their plane words where there is room (every other buffer
     // of the call is in place), so that the bands above find all their halves there or in the
     // resident table and run in odd mode too: M(10^16) with 6e9 of 2.27e10 values resident
-    // 54.2 -> 43.4 ms.
+    // 54.2 -> 43.4 ms.  At most half of what the budget has left: a resident limit is set to
+    // hold little.
     const int64_t w_res = (sp.nseg_res - sp.dense_segs) * (S / 64);
     int64_t kept = 0;  // bands [0, kept)
     if (odd_ok) {
@@ -868,7 +869,10 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
             if (vlo >= sp.u_total / 2) break;
             ++kept;
         }
-        if (kept == sp.nbands || ensure(c, c->kplanes, (size_t)kept * (size_t)sp.band_segs * (size_t)(S / 64) * 16)) kept = 0;
+        const uint64_t need = (uint64_t)kept * (uint64_t)sp.band_segs * (uint64_t)(S / 64) * 16;
+        const uint64_t others = c->held - c->kplanes.cap;
+        const bool room = !c->budget || (others < c->budget && need <= (c->budget - others) / 2);
+        if (kept == sp.nbands || !room || ensure(c, c->kplanes, (size_t)need)) kept = 0;
         if (kept) {
             ao.hsplit = w_res;
             ao.hplanes2 = (const ulonglong2*)c->kplanes.p - w_res;
