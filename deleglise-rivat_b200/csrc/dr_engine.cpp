@@ -949,6 +949,9 @@ struct WindowWork {
     std::vector<uint32_t> w;  // window of each item
     std::vector<float> cost;  // its lookups, about
     std::vector<TileWinTask> tasks;
+    // one copy to the device: the items, then the tasks on a 16-byte boundary
+    size_t item_bytes() const { return (items.size() * sizeof(TileWinItem) + 15) & ~size_t(15); }
+    size_t bytes() const { return item_bytes() + tasks.size() * sizeof(TileWinTask); }
 };
 
 // Items of the window kernel for one query: for each window the blocks whose windows include
@@ -1048,6 +1051,29 @@ void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P
     out.tasks = std::move(sorted);
 }
 
+// Room for the window kernel's work (none asked for: true).  All or nothing: a part that does
+// not fit gives back what the others took.
+bool reserve_windows(dr_ctx* c, u64 blocks, const WindowWork& ww) {
+    if (ww.tasks.empty()) return true;
+    bool ok = !ensure(c, c->groups, (size_t)blocks * 2 * sizeof(WinGroup)) && !ensure(c, c->titems, ww.bytes());
+    if (ok && c->tstage_cap < ww.bytes()) {  // the previous call's copies have completed (it synchronised)
+        if (c->capturing) return false;      // the eager pass found room: the same bytes again
+        if (c->tstage) cudaFreeHost(c->tstage);
+        c->tstage = nullptr;
+        c->tstage_cap = 0;
+        const size_t cap = ww.bytes() + ww.bytes() / 4;
+        ok = cudaMallocHost((void**)&c->tstage, cap) == cudaSuccess;
+        if (ok) c->tstage_cap = cap;
+        else cudaGetLastError();
+    }
+    if (!ok && !c->capturing) {
+        drop_graphs(c);  // a kept graph may read them
+        release(c, c->groups);
+        release(c, c->titems);
+    }
+    return ok;
+}
+
 int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, const dr_params* tuning,
                     int* launches_out, const StreamPlan* sp = nullptr) {
     int rc;
@@ -1097,19 +1123,6 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         witems = s1win_items(q, (int)i);
         if (witems.empty()) q.win = q.win_max = 0;
     }
-    // the window kernel's work
-    WindowWork ww;
-    if (witems.empty() && blocks > 0) {
-        window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
-        // buffers beyond what the call needs anyway: without room for them the tile kernel
-        // takes these lookups too
-        if (!ww.tasks.empty() && (ensure(c, c->groups, (size_t)blocks * 2 * sizeof(WinGroup)) ||
-                                  ensure(c, c->titems, ww.items.size() * sizeof(TileWinItem) + 16 +
-                                                           ww.tasks.size() * sizeof(TileWinTask)))) {
-            for (QueryDev& q : qs) q.twin_max = 0;
-            ww.tasks.clear();
-        }
-    }
     const int64_t invw_count = c->t_mu_limit / 6 + 1;  // every S2 j <= A <= mu_limit
     if ((rc = ensure(c, c->queries, (size_t)nq * sizeof(QueryDev)))) return rc;
     const size_t res_words = (size_t)nq * (3 + kCountsPerQuery) + 4;
@@ -1131,6 +1144,14 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     }
     if ((rc = ensure(c, c->inv, (size_t)(inv_limit + 1) * 8))) return rc;
     if ((rc = ensure(c, c->invw, (size_t)invw_count * 16))) return rc;
+    // The window kernel's work.  Its buffers come last: where the budget, the device or pinned
+    // memory has no room for them, they are given up and the tile kernel takes these lookups too.
+    WindowWork ww;
+    if (witems.empty() && blocks > 0) window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
+    if (!reserve_windows(c, blocks, ww)) {
+        for (QueryDev& q : qs) q.twin_max = 0;
+        ww = WindowWork{};
+    }
     const size_t need_pinned = (size_t)nq * (3 + kCountsPerQuery) + 2;
     if (c->pinned_cap < need_pinned) {
         if (c->capturing) return fail(DR_ERR_ARG, "internal: result buffer growth during graph capture");
@@ -1142,19 +1163,10 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     }
     const void* sq = stage_put(c, qs.data(), (size_t)nq * sizeof(QueryDev));
     if (!sq) return fail(DR_ERR_NOMEM, "internal: staging area too small");
-    const size_t item_bytes = (ww.items.size() * sizeof(TileWinItem) + 15) & ~size_t(15);
+    const size_t item_bytes = ww.item_bytes();
     const bool windows = !ww.tasks.empty();
-    c->tstage_used = windows ? item_bytes + ww.tasks.size() * sizeof(TileWinTask) : 0;
+    c->tstage_used = windows ? ww.bytes() : 0;
     if (windows) {
-        if (c->tstage_cap < c->tstage_used) {  // the previous call's copies have completed (it synchronised)
-            if (c->capturing) return fail(DR_ERR_ARG, "internal: staging growth during graph capture");
-            if (c->tstage) cudaFreeHost(c->tstage);
-            c->tstage = nullptr;
-            c->tstage_cap = 0;
-            const size_t cap = c->tstage_used + c->tstage_used / 4;
-            CU(cudaMallocHost((void**)&c->tstage, cap));
-            c->tstage_cap = cap;
-        }
         std::memcpy(c->tstage, ww.items.data(), ww.items.size() * sizeof(TileWinItem));
         std::memcpy(c->tstage + item_bytes, ww.tasks.data(), ww.tasks.size() * sizeof(TileWinTask));
     }
