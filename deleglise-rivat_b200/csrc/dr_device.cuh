@@ -205,11 +205,11 @@ struct QueryDev {
     i64 N;          // X / u
     i64 nc;         // candidates k <= N coprime to 6
     u64 slot_base;  // first global evaluation slot of this query
-    u64 blk_base;   // first 32-candidate block of this query
-    u64 win;        // S1 window length W (a power of two; 0: no windowed S1)
-    u64 win_max;    // windows w < win_max lie in the dense tier ((w+1)*W <= u_dense < 2^31)
     u64 inv_limit;  // largest tabulated S1 reciprocal 1/n
-    u64 twin_max;   // windows of kTileWin table values the window kernel may use (0: none)
+    uint32_t blk_base;  // first 32-candidate block of this query
+    uint32_t win;       // S1 window length W (a power of two; 0: no windowed S1)
+    uint32_t win_max;   // windows w < win_max lie in the dense tier ((w+1)*W <= u_dense < 2^31)
+    uint32_t twin_max;  // windows of kTileWin table values the window kernel may use (0: none)
 };
 
 #ifndef DRB_WIN_MIN

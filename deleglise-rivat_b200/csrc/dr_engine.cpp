@@ -1014,7 +1014,7 @@ void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P
     if (total < kWinMinLookups) return;
     const double task = std::max(total / (sm_count * 12.0), 524288.0);  // a dozen to a CTA
     for (size_t i = 0; i < qs.size(); ++i)
-        if ((qs[i].twin_max = window_limit(X[i], P[i], u_dense))) window_items(qs[i], (int)i, task, out);
+        if ((qs[i].twin_max = (uint32_t)window_limit(X[i], P[i], u_dense))) window_items(qs[i], (int)i, task, out);
     const size_t n = out.items.size();
     if (qs.size() > 1) {
         std::vector<uint32_t> at(n);
@@ -1049,6 +1049,14 @@ void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P
     std::vector<TileWinTask> sorted;
     for (uint32_t i : at) sorted.push_back(out.tasks[i]);
     out.tasks = std::move(sorted);
+}
+
+// Room for n op counts, their prefix and the scan's scratch.
+int reserve_ops(dr_ctx* c, u64 n) {
+    int rc = ensure(c, c->ops, (size_t)std::max<u64>(n, 1) * 8);
+    if (!rc) rc = ensure(c, c->prefix, (size_t)(n + 1) * 8);
+    if (!rc) rc = ensure(c, c->scan_tmp, scan_u64_tmp_elems(n) * 8);
+    return rc;
 }
 
 // Room for the window kernel's work (none asked for: true).  All or nothing: a part that does
@@ -1089,7 +1097,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         q.N = (X[i] <= c->t_u_total) ? 0 : X[i] / P[i].u_total;
         q.nc = num_candidates(q.N);
         q.slot_base = slots;
-        q.blk_base = blocks;
+        q.blk_base = (uint32_t)blocks;
         slots += 2 * (u64)q.nc;
         blocks += (u64)(q.nc + 31) / 32;
         if (q.N > 0) {
@@ -1117,9 +1125,9 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         const int wl = P[i].s1_window_log2;
         if (nq != 1 || q.N <= 0 || wl < 12 || wl > 16) continue;
         const int64_t W = int64_t(1) << wl;
-        q.win_max = (u64)(std::min<int64_t>(c->t_u_dense, (int64_t(1) << 31) - 1) / W);
+        q.win_max = (uint32_t)(std::min<int64_t>(c->t_u_dense, (int64_t(1) << 31) - 1) / W);
         if (q.win_max < 2) continue;
-        q.win = (u64)W;
+        q.win = (uint32_t)W;
         witems = s1win_items(q, (int)i);
         if (witems.empty()) q.win = q.win_max = 0;
     }
@@ -1130,24 +1138,29 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     u64* const acc = (u64*)c->acc.p;
     i64* const counts = (i64*)(acc + 3 * nq);
     u64* const ticket = acc + (size_t)nq * (3 + kCountsPerQuery);
-    // ops per slot for the sums kernel (the windowed S1, the bands, what the tile kernel
-    // leaves), per (block, e) for the tile kernel
-    const u64 n_ops = !witems.empty() || sp || rest ? std::max(slots, 2 * blocks) : 2 * blocks;
-    if ((rc = ensure(c, c->ops, (size_t)std::max<u64>(n_ops, 1) * 8))) return rc;
-    if ((rc = ensure(c, c->prefix, (size_t)(n_ops + 1) * 8))) return rc;
-    if (witems.empty() && (rc = ensure(c, c->tgroups, (size_t)std::max<u64>(2 * blocks, 1) * sizeof(TileGroup)))) return rc;
     if ((rc = ensure(c, c->slots, (size_t)std::max<u64>(slots, 1) * sizeof(SlotDesc)))) return rc;
-    if ((rc = ensure(c, c->scan_tmp, scan_u64_tmp_elems(n_ops) * 8))) return rc;
     if (!witems.empty()) {
         if ((rc = ensure(c, c->wdesc, (size_t)std::max<u64>(slots, 1) * sizeof(S1WinDesc)))) return rc;
         if ((rc = ensure(c, c->witems, witems.size() * sizeof(S1WinItem)))) return rc;
     }
     if ((rc = ensure(c, c->inv, (size_t)(inv_limit + 1) * 8))) return rc;
     if ((rc = ensure(c, c->invw, (size_t)invw_count * 16))) return rc;
+    // ops per slot for the sums kernel (the windowed S1, the bands, what the tile kernel
+    // leaves), per (block, e) for the tile kernel.  Where the tile kernel's records do not fit
+    // beside them, ops per slot and the sums kernel for everything: a block holds up to 64 slots
+    // (16 bytes each; 352 for the records and the ops of the block), so only calls that need the
+    // ops per slot anyway, or whose queries have a few candidates each, come to that.
+    bool tiles = witems.empty();  // the windowed S1 leaves every other lookup to the sums kernel
+    const bool per_slot = !tiles || sp || rest;
+    if ((rc = reserve_ops(c, per_slot ? slots : 2 * blocks))) return rc;
+    if (tiles && ensure(c, c->tgroups, (size_t)std::max<u64>(2 * blocks, 1) * sizeof(TileGroup))) {
+        tiles = false;
+        if (!per_slot && (rc = reserve_ops(c, slots))) return rc;
+    }
     // The window kernel's work.  Its buffers come last: where the budget, the device or pinned
     // memory has no room for them, they are given up and the tile kernel takes these lookups too.
     WindowWork ww;
-    if (witems.empty() && blocks > 0) window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
+    if (tiles && blocks > 0) window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
     if (!reserve_windows(c, blocks, ww)) {
         for (QueryDev& q : qs) q.twin_max = 0;
         ww = WindowWork{};
@@ -1190,7 +1203,6 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     const TableView T = view_of(c);
     const int qn = (int)nq;
     const S1Band band{0, sp ? (u64)sp->u_res : ~0ull, 0};
-    const bool tiles = !sw;  // the windowed S1 leaves every other lookup to the sums kernel
     CU(record_event(c, 2));
     CU(cudaMemcpyAsync(c->queries.p, sq, (size_t)nq * sizeof(QueryDev), cudaMemcpyHostToDevice, c->stream));
     CU(cudaMemsetAsync(acc, 0, res_words * 8, c->stream));
