@@ -858,8 +858,10 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
     // The bands below u_total/2 keep their plane words where there is room (every other buffer
     // of the call is in place), so that the bands above find all their halves there or in the
     // resident table and run in odd mode too: M(10^16) with 6e9 of 2.27e10 values resident
-    // 54.2 -> 43.4 ms.  At most half of what the budget has left: a resident limit is set to
-    // hold little.
+    // 54.2 -> 42.9 ms.  A resident limit is set to hold little, so they take at most half of what
+    // the limit's own table and band buffers take (the limit still bounds the call) and half of
+    // what the budget has left.  They stay until the limit changes: freed and allocated anew in
+    // each call they cost 0.4 to 4 ms (M(10^16) 42.9 -> 44.5 ms, M(10^14) 4.2 -> 6 to 8 ms).
     const int64_t w_res = (sp.nseg_res - sp.dense_segs) * (S / 64);
     int64_t kept = 0;  // bands [0, kept)
     if (odd_ok) {
@@ -870,8 +872,11 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
             ++kept;
         }
         const uint64_t need = (uint64_t)kept * (uint64_t)sp.band_segs * (uint64_t)(S / 64) * 16;
+        const uint64_t limit = 2 * (uint64_t)sp.u_dense +
+                               20 * (uint64_t)(w_res + sp.band_segs * (int64_t)(S / 64));
         const uint64_t others = c->held - c->kplanes.cap;
-        const bool room = !c->budget || (others < c->budget && need <= (c->budget - others) / 2);
+        const bool room = need <= limit / 2 &&
+                          (!c->budget || (others < c->budget && need <= (c->budget - others) / 2));
         if (kept == sp.nbands || !room || ensure(c, c->kplanes, (size_t)need)) kept = 0;
         if (kept) {
             ao.hsplit = w_res;
@@ -1535,6 +1540,10 @@ int dr_ctx_destroy(dr_ctx* c) {
 int dr_ctx_set_resident_limit(dr_ctx* c, int64_t u_resident, int64_t band_values) {
     if (!c) return fail(DR_ERR_ARG, "ctx is NULL");
     if (u_resident < 0 || band_values < 0) return fail(DR_ERR_ARG, "u_resident and band_values must be >= 0");
+    if (c->kplanes.p && (u_resident != c->u_resident || band_values != c->band_values)) {
+        CU(cudaSetDevice(c->device));
+        release(c, c->kplanes);  // sized for the old limit; no call is in flight
+    }
     c->u_resident = u_resident;
     c->band_values = band_values;
     return DR_OK;

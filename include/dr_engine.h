@@ -107,10 +107,11 @@ int dr_ctx_set_hbm_budget(dr_ctx *ctx, uint64_t bytes);
  * segment of the compressed tier, at least one segment above u_dense) in memory; the
  * compressed tier above is sieved band by band, band_values values at a time (0: as
  * many as the resident compressed tier holds), and after each band the S1 lookups
- * whose quotient falls in it are summed.  Where half of what the budget has left takes
- * them, the plane words of the bands below u_total/2 (0.25 bytes a value) are kept, which
- * halves the work of the bands above.  M(X) and the C/S1/S2 checksums are those of the
- * whole table.  Needs X > u_total and mu_limit <= u_res; batches never stream.
+ * whose quotient falls in it are summed.  Where they take at most half of what the
+ * resident table and the band buffers take, and half of what the budget has left, the
+ * plane words of the bands below u_total/2 (0.25 bytes a value) are kept, which halves
+ * the work of the bands above; they are given back when the limit changes.  M(X) and the
+ * C/S1/S2 checksums are those of the whole table.  Needs X > u_total and mu_limit <= u_res; batches never stream.
  * u_resident = 0 (the default) holds every table whole.  The bands' build and lookups
  * count in dr_stats.sums_ms (split out in band_table_ms and band_sums_ms). */
 int dr_ctx_set_resident_limit(dr_ctx *ctx, int64_t u_resident, int64_t band_values);
