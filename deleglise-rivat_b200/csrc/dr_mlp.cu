@@ -149,6 +149,11 @@ __global__ void mlp_reduce_kernel(const float* __restrict__ G, const float* __re
 // latency: by timing with a half left out, 4.9 us a step for the examples (chains of 64
 // dependent FMAs), 5.3 us for the parameters (exchange through L2 and the chain of B
 // additions), 0.5 us for a barrier.
+//
+// Chunk and side-by-side count were chosen at a tuner's training set of 305 examples (one chunk,
+// one round of 16 x 8 x 3); larger sets take several of each.  100 steps, five launches a step ->
+// here: 1 example 1.66 -> 0.62 ms, 32 2.03 -> 0.70, 385 4.33 -> 1.72, 1000 9.27 -> 3.41, 4096
+// 34.8 -> 11.8.  Where a device has no room for the cluster, dr_mlp_train runs the launches.
 constexpr int kTrainCtas = 16, kTrainThreads = 512, kTrainSlots = kTrainThreads / kHid;
 constexpr int kTrainChunk = 320;  // examples staged at a time in the second half
 constexpr int kTrainIlp = 3;      // examples a slot runs side by side (independent FMA chains)
@@ -421,6 +426,22 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
     }
 }
 
+// The same update step by step, after mlp_forward_kernel, mlp_backward_kernel and
+// mlp_reduce_kernel: step s of a call (the counter on the device moves when the call ends).
+__global__ void mlp_adam_kernel(float* __restrict__ P, const float* __restrict__ grad, float* __restrict__ m,
+                                float* __restrict__ v, const float* __restrict__ step, int s, float lr) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= kParams) return;
+    const float t = *step + (float)(s + 1);
+    AdamState a = {P[p], m[p], v[p]};
+    adam_step(a, grad[p], lr, 1.f - powf(0.9f, t), 1.f - powf(0.999f, t));
+    P[p] = a.p;
+    m[p] = a.m;
+    v[p] = a.v;
+}
+
+__global__ void mlp_step_advance(float* step, int steps) { *step += (float)steps; }
+
 }  // namespace
 
 struct dr_mlp {
@@ -434,6 +455,7 @@ struct dr_mlp {
     float* loss = nullptr;
     float *x = nullptr, *t = nullptr, *h1 = nullptr, *h2 = nullptr, *y = nullptr, *G = nullptr, *sq = nullptr;
     int cap = 0;  // examples the work buffers hold
+    int clusters = -1;  // clusters of mlp_train_kernel the device holds at once (-1: not asked yet)
 };
 
 namespace {
@@ -456,6 +478,32 @@ int mlp_reserve(dr_mlp* n, int B) {
     for (int i = 0; i < 7; ++i) MCU(cudaMalloc(bufs[i], sz[i] * sizeof(float)));
     n->cap = B;
     return DR_OK;
+}
+
+// Launch configuration of mlp_train_kernel.  False where the device does not hold a cluster of 16
+// such CTAs at once (a slice of a GPU, no GPC with 16 free SMs): training then runs step by step.
+bool mlp_train_config(dr_mlp* n, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at) {
+    cfg->gridDim = dim3(kTrainCtas);
+    cfg->blockDim = dim3(kTrainThreads);
+    cfg->dynamicSmemBytes = sizeof(TrainShared);
+    cfg->stream = n->stream;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = kTrainCtas;
+    at->val.clusterDim.y = at->val.clusterDim.z = 1;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+    if (n->clusters < 0) {
+        const bool ok = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(TrainShared)) == cudaSuccess &&
+                        cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                            cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n->clusters, mlp_train_kernel, cfg) == cudaSuccess;
+        if (!ok) {
+            n->clusters = 0;
+            cudaGetLastError();
+        }
+    }
+    return n->clusters > 0;
 }
 
 // Training domain of the shipped network: X in [10^10, 10^16], budgets of
@@ -607,28 +655,31 @@ int dr_mlp_grad(dr_mlp* n, const float* x, const float* t, int64_t B, float* gra
     return DR_OK;
 }
 
-// Full-batch Adam: `steps` updates on the B examples in one launch.
-int dr_mlp_train(dr_mlp* n, const float* x, const float* t, int64_t B, int steps, float lr, float* final_loss) {
+}  // extern "C"
+
+// Full-batch Adam: `steps` updates on the B examples, in one cluster launch or step by step.
+static int mlp_train(dr_mlp* n, const float* x, const float* t, int64_t B, int steps, float lr, float* final_loss,
+                     bool one_launch) {
     if (!n || !x || !t || B < 1 || B > kMaxBatch || steps < 0) return mlp_fail(DR_ERR_ARG, "dr_mlp_train: bad argument");
     int rc = mlp_reserve(n, (int)B);
     if (rc) return rc;
     MCU(cudaMemcpyAsync(n->x, x, B * kIn * sizeof(float), cudaMemcpyHostToDevice, n->stream));
     MCU(cudaMemcpyAsync(n->t, t, B * kOut * sizeof(float), cudaMemcpyHostToDevice, n->stream));
-    if (steps > 0) {
-        MCU(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)sizeof(TrainShared)));
-        MCU(cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(kTrainCtas);
-        cfg.blockDim = dim3(kTrainThreads);
-        cfg.dynamicSmemBytes = sizeof(TrainShared);
-        cfg.stream = n->stream;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = kTrainCtas;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    if (steps > 0 && one_launch) one_launch = mlp_train_config(n, &cfg, at);
+    if (steps > 0 && !one_launch) {
+        for (int s = 0; s < steps; ++s) {
+            mlp_forward_kernel<<<(unsigned)B, 64, 0, n->stream>>>(n->P, n->x, (int)B, n->h1, n->h2, n->y);
+            mlp_backward_kernel<<<(unsigned)B, 64, 0, n->stream>>>(n->P, n->x, n->t, n->h1, n->h2, n->y, (int)B, n->G,
+                                                                    n->sq);
+            mlp_reduce_kernel<<<(kParams + 255) / 256, 256, 0, n->stream>>>(n->G, n->sq, (int)B, n->grad, n->loss);
+            mlp_adam_kernel<<<(kParams + 255) / 256, 256, 0, n->stream>>>(n->P, n->grad, n->m, n->v, n->step, s, lr);
+        }
+        mlp_step_advance<<<1, 1, 0, n->stream>>>(n->step, steps);
+        MCU(cudaGetLastError());
+    }
+    if (steps > 0 && one_launch) {
         // the per-example gradients' buffer (B x kParams) holds d1, d2 and dy here
         float *d1 = n->G, *d2 = n->G + (size_t)B * kHid, *dy = n->G + 2 * (size_t)B * kHid;
         MCU(cudaLaunchKernelEx(&cfg, mlp_train_kernel, n->P, n->m, n->v, n->step, (const float*)n->x,
@@ -639,6 +690,17 @@ int dr_mlp_train(dr_mlp* n, const float* x, const float* t, int64_t B, int steps
     MCU(cudaStreamSynchronize(n->stream));
     if (final_loss) *final_loss = l;
     return DR_OK;
+}
+
+extern "C" {
+
+int dr_mlp_train(dr_mlp* n, const float* x, const float* t, int64_t B, int steps, float lr, float* final_loss) {
+    return mlp_train(n, x, t, B, steps, lr, final_loss, true);
+}
+
+int dr_debug_mlp_train_steps(dr_mlp* n, const float* x, const float* t, int64_t B, int steps, float lr,
+                             float* final_loss) {
+    return mlp_train(n, x, t, B, steps, lr, final_loss, false);
 }
 
 // Engine parameters for X from the network's outputs (no check, no fallback).

@@ -160,6 +160,8 @@ def lib():
                                   ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float)]),
             "dr_mlp_train": (i32, [vp, ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float), i64, i32,
                                    ctypes.c_float, ctypes.POINTER(ctypes.c_float)]),
+            "dr_debug_mlp_train_steps": (i32, [vp, ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float), i64,
+                                               i32, ctypes.c_float, ctypes.POINTER(ctypes.c_float)]),
             "dr_tuner_features": (i32, [i64, u64, i32, i32, ctypes.POINTER(ctypes.c_float)]),
             "dr_tuner_params": (i32, [i64, ctypes.POINTER(ctypes.c_float), P]),
             "dr_tuner_propose": (i32, [vp, i64, u64, i32, i32, P, ctypes.POINTER(i32)]),
@@ -187,7 +189,7 @@ def exported_symbols() -> list:
         "dr_table_build_noalloc", "dr_autotune_batch",
         "dr_mlp_create", "dr_mlp_destroy", "dr_mlp_num_params", "dr_mlp_set_weights", "dr_mlp_get_weights",
         "dr_mlp_forward", "dr_mlp_grad", "dr_mlp_train", "dr_tuner_features", "dr_tuner_params", "dr_tuner_propose",
-        "dr_measure_peaks", "dr_debug_sieve_plan", "dr_debug_stream_plan",
+        "dr_measure_peaks", "dr_debug_sieve_plan", "dr_debug_stream_plan", "dr_debug_mlp_train_steps",
     ]
 
 

@@ -173,7 +173,8 @@ int dr_mlp_get_weights(dr_mlp *mlp, float *w, int64_t count);
 int dr_mlp_forward(dr_mlp *mlp, const float *x, int64_t B, float *y);
 /* Gradient of the mean squared error over B examples (no update). */
 int dr_mlp_grad(dr_mlp *mlp, const float *x, const float *t, int64_t B, float *grad, float *loss);
-/* `steps` full-batch Adam updates (one kernel launch). */
+/* `steps` full-batch Adam updates (one launch of a 16-CTA cluster; where the device has no
+ * room for one, the same updates step by step). */
 int dr_mlp_train(dr_mlp *mlp, const float *x, const float *t, int64_t B, int steps, float lr,
                  float *final_loss);
 int dr_tuner_features(int64_t X, uint64_t hbm_budget, int sm_count, int batch, float *out4);
@@ -225,6 +226,10 @@ int64_t dr_debug_sieve_plan(int64_t u_total, int64_t u_dense, int32_t segment_lo
  * count (0: nothing streams) or a negative DR_ERR_* code.  Needs no GPU. */
 int64_t dr_debug_stream_plan(int64_t u_total, int64_t u_dense, int32_t segment_log2, int64_t u_resident,
                              int64_t band_values, int64_t *u_res, int64_t *out, int64_t cap);
+/* dr_mlp_train by its step-by-step route on any device -- test support, no counterpart in
+ * the reference: the same weights and loss, bit for bit. */
+int dr_debug_mlp_train_steps(dr_mlp *mlp, const float *x, const float *t, int64_t B, int steps, float lr,
+                             float *final_loss);
 
 /* Measured throughput ceilings of the units this engine's kernels are bound by
  * (measurement support for bench.py; no counterpart in the reference).  Each is
