@@ -88,6 +88,7 @@ struct dr_ctx {
     int64_t u_resident = 0, band_values = 0;
     std::vector<cudaEvent_t> bev;  // band timing: start, then per band after its build and after its sums
     int64_t last_bands = 0;        // bands the enqueued call streams
+    int table_launches = 0;        // kernels of the last table build
     // query buffers
     DevBuf queries, ops, prefix, scan_tmp, misc, inv, invw, wdesc, witems, slots;
     DevBuf acc;             // results: 3 sums and kCountsPerQuery counters per query, then 4 words of work queues
@@ -504,19 +505,18 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
 
     CU(record_event(c, 0));
     CU(cudaMemsetAsync(c->wheel.p, 0, (size_t)wheel_groups * 16, c->stream));
-    int launches = 3;
+    int launches = 0;
     if (a.sq_off) {
         CU(cudaMemsetAsync(c->sq_cnt.p, 0, (size_t)nseg * 8, c->stream));
         CU(cudaMemsetAsync(c->sq_cur.p, 0, (size_t)nseg * 8, c->stream));
-        launch_sq_bucket_count(a.primes, a.sqC_first, (int)pr.size(), 0, u_total, u_dense,
-                               dense_segs, lgS, 0, (u64*)c->sq_cnt.p, c->stream);
-        launch_scan_u64((const u64*)c->sq_cnt.p, (u64*)c->sq_off.p, (u64)nseg, (u64*)c->sq_tmp.p,
-                        scan_u64_tmp_elems((u64)nseg), c->stream);
-        launch_sq_bucket_fill(a.primes, a.sqC_first, (int)pr.size(), 0, u_total, u_dense,
-                              dense_segs, lgS, 0, (const u64*)c->sq_off.p, (u64*)c->sq_cur.p, (uint32_t*)c->sq_pos.p,
-                              c->stream);
+        launches += launch_sq_bucket_count(a.primes, a.sqC_first, (int)pr.size(), 0, u_total, u_dense, dense_segs,
+                                           lgS, 0, (u64*)c->sq_cnt.p, c->stream);
+        launches += launch_scan_u64((const u64*)c->sq_cnt.p, (u64*)c->sq_off.p, (u64)nseg, (u64*)c->sq_tmp.p,
+                                    scan_u64_tmp_elems((u64)nseg), c->stream);
+        launches += launch_sq_bucket_fill(a.primes, a.sqC_first, (int)pr.size(), 0, u_total, u_dense, dense_segs, lgS,
+                                          0, (const u64*)c->sq_off.p, (u64*)c->sq_cur.p, (uint32_t*)c->sq_pos.p,
+                                          c->stream);
         CU(cudaGetLastError());
-        launches += 5;
     }
     // Each sieve launch covers the segments [begin, end) in order.  Once it is done, the
     // side stream scans their Mobius sums (continuing from the segments before) and
@@ -535,11 +535,12 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
                      block, l.odd ? smem_o : smem_f, c->stream);
         CU(cudaGetLastError());
         if (plan.size() == 1) {  // nothing to overlap: no side stream
-            launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, 0, l.end, 1024, c->stream);
-            launch_fixup_range((int16_t*)c->dM.p, u_dense, S, (const int32_t*)c->seg_off.p, (int32_t*)c->ckpt.p,
-                               nwords, dense_segs, 0, l.end, c->sm_count * 16, c->stream);
+            launches += launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, 0, l.end, 1024,
+                                              c->stream);
+            launches += launch_fixup_range((int16_t*)c->dM.p, u_dense, S, (const int32_t*)c->seg_off.p,
+                                           (int32_t*)c->ckpt.p, nwords, dense_segs, 0, l.end, c->sm_count * 16,
+                                           c->stream);
             CU(cudaGetLastError());
-            launches += 2;
             break;
         }
         if (forks < dr_ctx::kForks - 1 || li + 1 == plan.size()) {
@@ -549,21 +550,21 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
             // SM's shared memory, not its threads); after the last one they are the tail
             // of the build and take the whole GPU
             const bool last = li + 1 == plan.size();
-            launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, fixed, l.end,
-                                  last ? 1024 : 256, c->side);
-            launch_fixup_range((int16_t*)c->dM.p, u_dense, S, (const int32_t*)c->seg_off.p, (int32_t*)c->ckpt.p,
-                               nwords, dense_segs, fixed, l.end, c->sm_count * (last ? 16 : 2), c->side);
+            launches += launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, fixed, l.end,
+                                              last ? 1024 : 256, c->side);
+            launches += launch_fixup_range((int16_t*)c->dM.p, u_dense, S, (const int32_t*)c->seg_off.p,
+                                           (int32_t*)c->ckpt.p, nwords, dense_segs, fixed, l.end,
+                                           c->sm_count * (last ? 16 : 2), c->side);
             CU(cudaGetLastError());
             fixed = l.end;
             ++forks;
-            launches += 2;
         }
     }
     if (plan.size() > 1) {
         CU(cudaEventRecord(c->join, c->side));
         CU(cudaStreamWaitEvent(c->stream, c->join, 0));
     }
-    launches += (int)plan.size() - 3;
+    launches += (int)plan.size();
     CU(record_event(c, 1));
 
     c->table_valid = true;
@@ -572,6 +573,7 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     c->t_mu_limit = mu_limit;
     c->t_nwords = nwords;
     c->t_S = S;
+    c->table_launches = launches;
     if (st) st->kernel_launches += launches;
     return DR_OK;
 }
@@ -904,23 +906,25 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
             const u64 nb = (u64)(c1 - c0);
             CU(cudaMemsetAsync(c->sq_cnt.p, 0, nb * 8, c->stream));
             CU(cudaMemsetAsync(c->sq_cur.p, 0, nb * 8, c->stream));
-            launch_sq_bucket_count(m.primes, m.sqC_first, (int)np, vlo, vhi, sp.u_dense, sp.dense_segs, lgS, c0,
-                                   (u64*)c->sq_cnt.p, c->stream);
-            launch_scan_u64((const u64*)c->sq_cnt.p, (u64*)c->sq_off.p, nb, (u64*)c->sq_tmp.p,
-                            scan_u64_tmp_elems(nb), c->stream);
-            launch_sq_bucket_fill(m.primes, m.sqC_first, (int)np, vlo, vhi, sp.u_dense, sp.dense_segs, lgS, c0,
-                                  (const u64*)c->sq_off.p, (u64*)c->sq_cur.p, (uint32_t*)c->sq_pos.p, c->stream);
+            *launches += launch_sq_bucket_count(m.primes, m.sqC_first, (int)np, vlo, vhi, sp.u_dense, sp.dense_segs,
+                                                lgS, c0, (u64*)c->sq_cnt.p, c->stream);
+            *launches += launch_scan_u64((const u64*)c->sq_cnt.p, (u64*)c->sq_off.p, nb, (u64*)c->sq_tmp.p,
+                                         scan_u64_tmp_elems(nb), c->stream);
+            *launches += launch_sq_bucket_fill(m.primes, m.sqC_first, (int)np, vlo, vhi, sp.u_dense, sp.dense_segs,
+                                               lgS, c0, (const u64*)c->sq_off.p, (u64*)c->sq_cur.p,
+                                               (uint32_t*)c->sq_pos.p, c->stream);
             m.sq_off = (const u64*)c->sq_off.p;
             m.sq_pos = (const uint32_t*)c->sq_pos.p;
-            *launches += 5;
         } else {
             m.sqC_first = (int)np;  // no bucketed hit in this band: squares thread-per-prime
         }
         launch_sieve(m, odd ? kSieveOdd : kSieveFull, (int)std::max<int64_t>(1, std::min<int64_t>(c1 - c0, odd ? sgrid_o : sgrid)), sp.block,
                      odd ? smem_o : smem, c->stream);
-        launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, c0, c1, 1024, c->stream);
-        launch_fixup_range((int16_t*)c->dM.p, sp.u_dense, S, (const int32_t*)c->seg_off.p, (int32_t*)c->bckpt.p,
-                           nwords_all, sp.dense_segs, c0, c1, c->sm_count * 16, c->stream, cword0);
+        *launches += launch_seg_scan_range((const int32_t*)c->seg_sum.p, (int32_t*)c->seg_off.p, c0, c1, 1024,
+                                           c->stream);
+        *launches += launch_fixup_range((int16_t*)c->dM.p, sp.u_dense, S, (const int32_t*)c->seg_off.p,
+                                        (int32_t*)c->bckpt.p, nwords_all, sp.dense_segs, c0, c1, c->sm_count * 16,
+                                        c->stream, cword0);
         CU(cudaGetLastError());
         CU(cudaEventRecord(c->bev[(size_t)(2 * b + 1)], c->stream));
         SumsArgs sa = base;
@@ -930,12 +934,12 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
         CU(cudaMemsetAsync(sa.ticket, 0, 8, c->stream));  // the work-queue counter (not the error flag)
         launch_plan(sa.queries, sa.nq, sa.T, sa.n_blocks, (u64*)c->ops.p, sa.acc, (i64*)(sa.acc + 3 * sa.nq), nullptr,
                     (SlotDesc*)c->slots.p, c->sm_count, c->stream, S1Band{(u64)vlo + 1, (u64)vhi, 1}, kPlanSlots);
-        launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, sa.n_slots, (u64*)c->scan_tmp.p,
-                        scan_u64_tmp_elems(sa.n_slots), c->stream);
+        *launches += launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, sa.n_slots, (u64*)c->scan_tmp.p,
+                                     scan_u64_tmp_elems(sa.n_slots), c->stream);
         launch_sums(sa, grid, 256, c->stream);
         CU(cudaGetLastError());
         CU(cudaEventRecord(c->bev[(size_t)(2 * b + 2)], c->stream));
-        *launches += 9;
+        *launches += 3;  // sieve, planning, sums
     }
     return DR_OK;
 }
@@ -1230,9 +1234,8 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
                     tiles ? kPlanTiles : kPlanSlots, tiles ? (TileGroup*)c->tgroups.p : nullptr,
                     windows ? (WinGroup*)c->groups.p : nullptr);
         const u64 n_scan = tiles ? 2 * blocks : slots;
-        launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, n_scan, (u64*)c->scan_tmp.p,
-                        scan_u64_tmp_elems(n_scan), c->stream);
-        launches += 5;
+        launches += 2 + launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, n_scan, (u64*)c->scan_tmp.p,
+                                        scan_u64_tmp_elems(n_scan), c->stream);
     }
     CU(cudaGetLastError());
     CU(record_event(c, 3));
@@ -1293,10 +1296,9 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
             // what the tile kernel leaves (y >= 2^51: a few small k of an X above it)
             launch_plan(sa.queries, qn, T, blocks, (u64*)c->ops.p, acc, counts, nullptr,
                         (SlotDesc*)c->slots.p, c->sm_count, c->stream, band, kPlanRest);
-            launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
-                            scan_u64_tmp_elems(slots), c->stream);
+            launches += 1 + launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, slots, (u64*)c->scan_tmp.p,
+                                            scan_u64_tmp_elems(slots), c->stream);
             CU(cudaMemsetAsync(ticket, 0, 8, c->stream));  // the work-queue counter (not the error flag)
-            launches += 4;
         }
         if (!tiles || rest) {
             launch_sums(sa, grid, 256, c->stream);
@@ -1419,7 +1421,7 @@ void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, 
     c->tstage = tsaved;
     c->tstage_cap = tsaved_cap;
     if (rc == DR_OK && graph && cudaGraphInstantiate(&g.exec, graph, 0) == cudaSuccess) {
-        g.launches = launches + 3;
+        g.launches = c->table_launches + launches;
         c->graphs.push_back(std::move(g));
     } else {
         if (g.stage) cudaFreeHost(g.stage);

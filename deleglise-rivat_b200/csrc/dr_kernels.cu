@@ -901,18 +901,19 @@ __global__ void sq_bucket_fill_kernel(const uint32_t* primes, int first, i64 vlo
     }
 }
 
-void launch_sq_bucket_count(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
-                            int lgS, i64 seg0, u64* counts, cudaStream_t s) {
-    if (n > first)
-        sq_bucket_count_kernel<<<n - first, 128, 0, s>>>(primes, first, vlo, vhi, u_dense, dense_segs, lgS, seg0,
-                                                         counts);
+int launch_sq_bucket_count(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
+                           int lgS, i64 seg0, u64* counts, cudaStream_t s) {
+    if (n <= first) return 0;
+    sq_bucket_count_kernel<<<n - first, 128, 0, s>>>(primes, first, vlo, vhi, u_dense, dense_segs, lgS, seg0, counts);
+    return 1;
 }
 
-void launch_sq_bucket_fill(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
-                           int lgS, i64 seg0, const u64* off, u64* cur, uint32_t* pos, cudaStream_t s) {
-    if (n > first)
-        sq_bucket_fill_kernel<<<n - first, 128, 0, s>>>(primes, first, vlo, vhi, u_dense, dense_segs, lgS, seg0, off,
-                                                        cur, pos);
+int launch_sq_bucket_fill(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
+                          int lgS, i64 seg0, const u64* off, u64* cur, uint32_t* pos, cudaStream_t s) {
+    if (n <= first) return 0;
+    sq_bucket_fill_kernel<<<n - first, 128, 0, s>>>(primes, first, vlo, vhi, u_dense, dense_segs, lgS, seg0, off, cur,
+                                                    pos);
+    return 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -941,8 +942,10 @@ void launch_seg_scan(const int32_t* in, int32_t* out, i64 n, cudaStream_t s) {
     seg_scan_kernel<<<1, 1024, 0, s>>>(in, out, 0, n);
 }
 
-void launch_seg_scan_range(const int32_t* in, int32_t* out, i64 b0, i64 b1, int threads, cudaStream_t s) {
-    if (b1 > b0) seg_scan_kernel<<<1, threads, 0, s>>>(in, out, b0, b1);
+int launch_seg_scan_range(const int32_t* in, int32_t* out, i64 b0, i64 b1, int threads, cudaStream_t s) {
+    if (b1 <= b0) return 0;
+    seg_scan_kernel<<<1, threads, 0, s>>>(in, out, b0, b1);
+    return 1;
 }
 
 // Adds the segment offsets to the dense prefix values of the 8-value groups [g0, g1)
@@ -971,8 +974,8 @@ __global__ void fixup_kernel(int16_t* dM, i64 u_dense, int lgS, const int32_t* s
 }
 
 // The fix-up of segments [b0, b1): their dense groups and their checkpoint words.
-void launch_fixup_range(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off, int32_t* ckpt, i64 nwords,
-                        i64 dense_segs, i64 b0, i64 b1, int blocks, cudaStream_t s, i64 cword0) {
+int launch_fixup_range(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off, int32_t* ckpt, i64 nwords,
+                       i64 dense_segs, i64 b0, i64 b1, int blocks, cudaStream_t s, i64 cword0) {
     int lgS = 0;  // S is a power of two (2^12 .. 2^18)
     while ((1 << lgS) < S) ++lgS;
     const i64 n8 = (u_dense + 7) / 8;
@@ -982,9 +985,10 @@ void launch_fixup_range(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off,
     // the last dense segment may end inside a group: its tail group belongs to it
     const i64 g1x = (b1 >= dense_segs) ? n8 : g1;
     const i64 work = std::max(g1x - g0, w1 - w0);
-    if (work <= 0) return;
+    if (work <= 0) return 0;
     const int grid = (int)std::max<i64>(1, std::min<i64>((work + 255) / 256, (i64)blocks));
     fixup_kernel<<<grid, 256, 0, s>>>(dM, u_dense, lgS, seg_off, ckpt, g0, g1x, w0, w1, dense_segs, cword0);
+    return 1;
 }
 
 void launch_fixup(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off, int32_t* ckpt, i64 nwords,
@@ -1328,19 +1332,20 @@ constexpr u64 kScanOneTiles = 4;
 
 size_t scan_u64_tmp_elems(u64 n) { return (size_t)((n + kScanTile - 1) / kScanTile) + 1; }
 
-void launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t, cudaStream_t s) {
+int launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t, cudaStream_t s) {
     const u64 ntiles = (n + kScanTile - 1) / kScanTile;
     if (ntiles == 0) {
         cudaMemsetAsync(out, 0, sizeof(u64), s);
-        return;
+        return 0;
     }
     if (ntiles <= kScanOneTiles) {
         scan_one<<<1, kScanBlock, 0, s>>>(in, n, out);
-        return;
+        return 1;
     }
     scan_tile_sums<<<(unsigned)ntiles, kScanBlock, 0, s>>>(in, n, tmp);
     scan_tile_offsets<<<1, kScanBlock, 0, s>>>(tmp, ntiles);
     scan_tile_apply<<<(unsigned)ntiles, kScanBlock, 0, s>>>(in, n, tmp, out, ntiles);
+    return 3;
 }
 
 // ---------------------------------------------------------------------------

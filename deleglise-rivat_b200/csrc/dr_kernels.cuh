@@ -119,9 +119,9 @@ void launch_sieve(const SieveArgs& a, int mode, int grid, int block, size_t smem
 // (p^2 > S: at most one per segment), counted per segment, then written per segment
 // in the order of off = exclusive scan of the counts (cur: zeroed cursors); bucket
 // arrays indexed by segment - seg0 (the whole table: vlo = seg0 = 0, vhi = u_total).
-void launch_sq_bucket_count(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
+int launch_sq_bucket_count(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
                             int lgS, i64 seg0, u64* counts, cudaStream_t s);
-void launch_sq_bucket_fill(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
+int launch_sq_bucket_fill(const uint32_t* primes, int first, int n, i64 vlo, i64 vhi, i64 u_dense, i64 dense_segs,
                            int lgS, i64 seg0, const u64* off, u64* cur, uint32_t* pos, cudaStream_t s);
 
 // Moduli with at least kItemDiv hits in the B bytes a segment sieves (m < B/kItemDiv)
@@ -151,11 +151,11 @@ size_t sieve_smem_bytes(int S, bool odd);
 void launch_seg_scan(const int32_t* in, int32_t* out, i64 n, cudaStream_t s);
 // The same for the segments [b0, b1) given out[b0] (written by the range before,
 // 0 for b0 = 0); also writes out[b1].  One CTA of `threads` (32 .. 1024, a multiple of 32).
-void launch_seg_scan_range(const int32_t* in, int32_t* out, i64 b0, i64 b1, int threads, cudaStream_t s);
+int launch_seg_scan_range(const int32_t* in, int32_t* out, i64 b0, i64 b1, int threads, cudaStream_t s);
 // Offsets added to the dense prefix and the checkpoints of the segments [b0, b1).
 // cword0: the compressed-tier word held in ckpt[0] (0 for a whole table, a band's
 // first word for a streamed band)
-void launch_fixup_range(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off, int32_t* ckpt, i64 nwords,
+int launch_fixup_range(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off, int32_t* ckpt, i64 nwords,
                         i64 dense_segs, i64 b0, i64 b1, int blocks, cudaStream_t s, i64 cword0 = 0);
 void launch_fixup(int16_t* dM, i64 u_dense, int S, const int32_t* seg_off, int32_t* ckpt, i64 nwords,
                   i64 dense_segs, int sm_count, cudaStream_t s);
@@ -174,7 +174,7 @@ void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u6
                  const S1Band& band, int mode, TileGroup* tgroups = nullptr, WinGroup* groups = nullptr);
 // Windowed S1 (window length win: a power of two, 2^12 .. 2^16).
 void launch_s1win(const S1WinArgs& a, u64 win, int sm_count, cudaStream_t s);
-void launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t tmp_elems, cudaStream_t s);
+int launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t tmp_elems, cudaStream_t s);
 size_t scan_u64_tmp_elems(u64 n);
 void launch_sums(const SumsArgs& a, int grid, int block, cudaStream_t s);
 // Work of the window kernel (dr_windows.cu).  A task, one CTA's: the items [i0, i1) of window
