@@ -1704,6 +1704,7 @@ int dr_mertens_batch(dr_ctx* c, const int64_t* X, int64_t count, const dr_params
         for (auto& g : c->graphs) {
             if (!same_batch(g, X, P.data(), count, tune)) continue;
             c->table_valid = false;  // the graph rebuilds the table in place
+            c->last_bands = 0;       // and streams nothing
             CU(cudaGraphLaunch(g.exec, c->stream));
             c->table_valid = true;
             c->t_u_total = ut;
