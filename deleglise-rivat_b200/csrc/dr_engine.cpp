@@ -134,6 +134,7 @@ struct dr_ctx {
         uint8_t* stage = nullptr;
         uint8_t* tstage = nullptr;
         int launches = 0;
+        size_t h2d_bytes = 0;  // what its copies read from the host
     };
     std::vector<Graph> graphs;  // replayable batch pipelines, most recent last
     bool graphs_enabled = true;
@@ -1415,6 +1416,7 @@ void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, 
         if (cudaStreamEndCapture(c->stream, &graph) != cudaSuccess) rc = DR_ERR_CUDA;
     }
     c->capturing = false;
+    g.h2d_bytes = c->stage_used + c->tstage_used;
     c->stage = saved;
     c->stage_cap = saved_cap;
     c->stage_used = saved_used;
@@ -1711,7 +1713,7 @@ int dr_mertens_batch(dr_ctx* c, const int64_t* X, int64_t count, const dr_params
             c->t_u_dense = ud;
             c->t_mu_limit = ml;
             c->t_nwords = (ut - ud + 63) / 64;
-            int rc = finish_queries(c, X, count, g.launches, stage_bytes_for(c->host_primes.size(), count), out, st);
+            int rc = finish_queries(c, X, count, g.launches, g.h2d_bytes, out, st);
             if (rc) return rc;
             if (st) st->total_ms = now_ms() - t0;
             return DR_OK;
