@@ -60,6 +60,17 @@ struct DevBuf {
     size_t cap = 0;
 };
 
+// The window kernel's work for one launch (window_work).
+struct WindowWork {
+    std::vector<TileWinItem> items;
+    std::vector<uint32_t> w;  // window of each item
+    std::vector<float> cost;  // its lookups, about
+    std::vector<TileWinTask> tasks;
+    // one copy to the device: the items, then the tasks on a 16-byte boundary
+    size_t item_bytes() const { return (items.size() * sizeof(TileWinItem) + 15) & ~size_t(15); }
+    size_t bytes() const { return item_bytes() + tasks.size() * sizeof(TileWinTask); }
+};
+
 double now_ms() {
     using namespace std::chrono;
     return duration<double, std::milli>(steady_clock::now().time_since_epoch()).count();
@@ -125,6 +136,7 @@ struct dr_ctx {
     // pinned copy of the window kernel's items and tasks (a graph owns its own)
     uint8_t* tstage = nullptr;
     size_t tstage_cap = 0, tstage_used = 0;
+    WindowWork ww;  // of the last enqueued call: a capture right after it takes the same
     bool capturing = false;
     struct Graph {
         std::vector<int64_t> X;
@@ -954,15 +966,6 @@ u64 window_limit(int64_t X, const dr_params& p, int64_t u_dense) {
     return (u64)(std::min(q, (double)std::min<int64_t>(u_dense, (int64_t(1) << 31) - 1)) / (double)kTileWin);
 }
 
-struct WindowWork {
-    std::vector<TileWinItem> items;
-    std::vector<uint32_t> w;  // window of each item
-    std::vector<float> cost;  // its lookups, about
-    std::vector<TileWinTask> tasks;
-    // one copy to the device: the items, then the tasks on a 16-byte boundary
-    size_t item_bytes() const { return (items.size() * sizeof(TileWinItem) + 15) & ~size_t(15); }
-    size_t bytes() const { return item_bytes() + tasks.size() * sizeof(TileWinTask); }
-};
 
 // Items of the window kernel for one query: for each window the blocks whose windows include
 // it (tile_windows), less the leading ones whose quotients all lie above it, in runs of at
@@ -1169,12 +1172,16 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     }
     // The window kernel's work.  Its buffers come last: where the budget, the device or pinned
     // memory has no room for them, they are given up and the tile kernel takes these lookups too.
-    WindowWork ww;
-    if (tiles && blocks > 0) window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
-    if (!reserve_windows(c, blocks, ww)) {
-        for (QueryDev& q : qs) q.twin_max = 0;
+    // A capture runs right after the same batch and takes its work: planned anew it cost 2 ms
+    // more in the first call of a 256-query batch.
+    WindowWork& ww = c->ww;
+    if (!c->capturing) {
         ww = WindowWork{};
+        if (tiles && blocks > 0) window_work(qs, X, P, c->t_u_dense, c->sm_count, ww);
     }
+    if (!tiles || !reserve_windows(c, blocks, ww)) ww = WindowWork{};
+    if (!ww.tasks.empty())
+        for (int64_t i = 0; i < nq; ++i) qs[(size_t)i].twin_max = (uint32_t)window_limit(X[i], P[i], c->t_u_dense);
     const size_t need_pinned = (size_t)nq * (3 + kCountsPerQuery) + 2;
     if (c->pinned_cap < need_pinned) {
         if (c->capturing) return fail(DR_ERR_ARG, "internal: result buffer growth during graph capture");
