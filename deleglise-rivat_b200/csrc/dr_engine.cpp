@@ -143,8 +143,8 @@ struct dr_ctx {
         std::vector<dr_params> P;
         dr_params tune;
         cudaGraphExec_t exec = nullptr;
-        uint8_t* stage = nullptr;
-        uint8_t* tstage = nullptr;
+        uint8_t* pin = nullptr;  // its own pinned staging: the call's, then the window work's
+        size_t pin_cap = 0;
         int launches = 0;
         size_t h2d_bytes = 0;  // what its copies read from the host
     };
@@ -157,8 +157,7 @@ namespace {
 void drop_graphs(dr_ctx* c) {
     for (auto& g : c->graphs) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
-        if (g.stage) cudaFreeHost(g.stage);
-        if (g.tstage) cudaFreeHost(g.tstage);
+        if (g.pin) cudaFreeHost(g.pin);
     }
     c->graphs.clear();
 }
@@ -1390,31 +1389,31 @@ int finish_queries(dr_ctx* c, const int64_t* X, int64_t nq, int launches, size_t
 // capture is not an error: the batch simply keeps running eagerly.
 void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, const dr_params& tune, int64_t ut,
                    int64_t ud, int64_t ml, size_t n_primes) {
-    if (c->graphs.size() >= 4) {
+    dr_ctx::Graph g;
+    if (c->graphs.size() >= 4) {  // the oldest makes room; its staging serves again
+        g.pin = c->graphs.front().pin;
+        g.pin_cap = c->graphs.front().pin_cap;
         if (c->graphs.front().exec) cudaGraphExecDestroy(c->graphs.front().exec);
-        if (c->graphs.front().stage) cudaFreeHost(c->graphs.front().stage);
-        if (c->graphs.front().tstage) cudaFreeHost(c->graphs.front().tstage);
         c->graphs.erase(c->graphs.begin());
     }
-    dr_ctx::Graph g;
     g.X.assign(X, X + nq);
     g.P.assign(P, P + nq);
     g.tune = tune;
-    const size_t need = stage_bytes_for(n_primes, nq);
-    if (cudaMallocHost((void**)&g.stage, need) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    if (c->tstage_used && cudaMallocHost((void**)&g.tstage, c->tstage_used) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFreeHost(g.stage);
-        return;
+    // one allocation for both: pinning costs milliseconds each time (4 to 15 ms for 1 MB here)
+    const size_t need = (stage_bytes_for(n_primes, nq) + 15) & ~size_t(15);
+    if (g.pin_cap < need + c->tstage_used) {
+        if (g.pin) cudaFreeHost(g.pin);
+        g.pin_cap = need + c->tstage_used + c->tstage_used / 4;
+        if (cudaMallocHost((void**)&g.pin, g.pin_cap) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
     }
     uint8_t *saved = c->stage, *tsaved = c->tstage;
     const size_t saved_cap = c->stage_cap, saved_used = c->stage_used, tsaved_cap = c->tstage_cap;
-    c->tstage = g.tstage;
-    c->tstage_cap = c->tstage_used;
-    c->stage = g.stage;
+    c->tstage = g.pin + need;
+    c->tstage_cap = g.pin_cap - need;
+    c->stage = g.pin;
     c->stage_cap = need;
     c->stage_used = 0;
     c->capturing = true;
@@ -1437,8 +1436,7 @@ void capture_graph(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq, 
         g.launches = c->table_launches + launches;
         c->graphs.push_back(std::move(g));
     } else {
-        if (g.stage) cudaFreeHost(g.stage);
-        if (g.tstage) cudaFreeHost(g.tstage);
+        cudaFreeHost(g.pin);
     }
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();

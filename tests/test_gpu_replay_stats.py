@@ -30,3 +30,18 @@ def test_host_bytes(X, n):
         again, st = e.mertens_batch(xs, p)
         assert again == out
         assert (st.h2d_bytes, st.d2h_bytes) == (first.h2d_bytes, first.d2h_bytes)
+
+
+def test_many_kept_batches():
+    """More batches than graphs are kept, of lengths that do and do not fit the staging of the
+    one that makes room; each replayed twice, with the others and single queries in between."""
+    p = dr_b200.default_params(10**15, dr_b200.POLICY_COMPRESSED)
+    batches = [[10**9 + k] * n for k, n in enumerate((3, 200, 5, 40))] + [[10**15 + k] * 3 for k in range(4)]
+    with dr_b200.Engine(0) as e:
+        want = [[e.mertens(x, p if x > 10**14 else None).M for x in xs] for xs in batches]
+        for _ in range(2):
+            for xs, w in zip(batches, want):
+                ps = [p] * len(xs) if xs[0] > 10**14 else None
+                for _ in range(2):
+                    assert e.mertens_batch(xs, ps)[0] == w
+                assert e.mertens(10**10).M == -33722
