@@ -1185,14 +1185,13 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     if (!tiles || !reserve_windows(c, blocks, ww)) ww = WindowWork{};
     if (!ww.tasks.empty())
         for (int64_t i = 0; i < nq; ++i) qs[(size_t)i].twin_max = (uint32_t)window_limit(X[i], P[i], c->t_u_dense);
-    const size_t need_pinned = (size_t)nq * (3 + kCountsPerQuery) + 2;
-    if (c->pinned_cap < need_pinned) {
+    if (c->pinned_cap < res_words) {
         if (c->capturing) return fail(DR_ERR_ARG, "internal: result buffer growth during graph capture");
         drop_graphs(c);
         if (c->pinned) cudaFreeHost(c->pinned);
         c->pinned = nullptr;
-        CU(cudaMallocHost((void**)&c->pinned, need_pinned * 8));
-        c->pinned_cap = need_pinned;
+        CU(cudaMallocHost((void**)&c->pinned, res_words * 8));
+        c->pinned_cap = res_words;
     }
     const void* sq = stage_put(c, qs.data(), (size_t)nq * sizeof(QueryDev));
     if (!sq) return fail(DR_ERR_NOMEM, "internal: staging area too small");
@@ -1243,7 +1242,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         launch_plan((const QueryDev*)c->queries.p, qn, T, blocks, (u64*)c->ops.p, acc, counts,
                     sw ? (S1WinDesc*)c->wdesc.p : nullptr, (SlotDesc*)c->slots.p, c->sm_count, c->stream, band,
                     tiles ? kPlanTiles : kPlanSlots, tiles ? (TileGroup*)c->tgroups.p : nullptr,
-                    windows ? (WinGroup*)c->groups.p : nullptr);
+                    windows ? (WinGroup*)c->groups.p : nullptr, ticket + 3);
         const u64 n_scan = tiles ? 2 * blocks : slots;
         launches += 2 + launch_scan_u64((const u64*)c->ops.p, (u64*)c->prefix.p, n_scan, (u64*)c->scan_tmp.p,
                                         scan_u64_tmp_elems(n_scan), c->stream);
@@ -1322,7 +1321,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
         }
     }
     CU(record_event(c, 4));
-    CU(cudaMemcpyAsync(c->pinned, acc, (res_words - 2) * 8, cudaMemcpyDeviceToHost, c->stream));
+    CU(cudaMemcpyAsync(c->pinned, acc, res_words * 8, cudaMemcpyDeviceToHost, c->stream));
     CU(record_event(c, 5));
     *launches_out = launches;
     return DR_OK;
@@ -1333,7 +1332,10 @@ int finish_queries(dr_ctx* c, const int64_t* X, int64_t nq, int launches, size_t
                    dr_stats* st) {
     CU(cudaStreamSynchronize(c->stream));
     CU(cudaGetLastError());
-    if (c->pinned[(size_t)nq * (3 + kCountsPerQuery) + 1])
+    const uint64_t* ticket = c->pinned + (size_t)nq * (3 + kCountsPerQuery);
+    if (ticket[3])
+        return fail(DR_ERR_DEVICE, "window kernel: %u planned lookups (mod 2^32) were not summed", (unsigned)ticket[3]);
+    if (ticket[1])
         return fail(DR_ERR_DEVICE, "sums kernel: op count of an evaluation disagreed with its plan");
     for (int64_t i = 0; i < nq; ++i) {
         uint64_t* a = c->pinned + 3 * i;
@@ -1363,7 +1365,7 @@ int finish_queries(dr_ctx* c, const int64_t* X, int64_t nq, int launches, size_t
         st->sieve_launches += 1;
         st->sums_launches += launches > 1 ? 1 : 0;
         st->h2d_bytes += (uint64_t)h2d_bytes;
-        st->d2h_bytes += (uint64_t)nq * (3 + kCountsPerQuery) * 8 + 16;
+        st->d2h_bytes += (uint64_t)nq * (3 + kCountsPerQuery) * 8 + 32;
         const uint64_t* cnt = c->pinned + (size_t)nq * 3;
         for (int64_t i = 0; i < nq; ++i) {
             const uint64_t* ci = cnt + (size_t)kCountsPerQuery * i;
@@ -2003,6 +2005,26 @@ int64_t dr_debug_stream_plan(int64_t u_total, int64_t u_dense, int32_t segment_l
         out[3 * b + 2] = band_odd(sp, out[3 * b], out[3 * b + 1]) ? 1 : 0;
     }
     return sp.nbands;
+}
+
+int64_t dr_debug_window_items(int64_t X, const dr_params* p, int32_t sm_count, int64_t* out, int64_t cap) {
+    if (X < 1 || !p || p->u_total < 1 || !(p->cx > 0.0) || sm_count < 1 || cap < 0 || (cap > 0 && !out))
+        return fail(DR_ERR_ARG, "dr_debug_window_items: bad arguments");
+    std::vector<QueryDev> q(1);
+    std::memset(&q[0], 0, sizeof(QueryDev));
+    q[0].X = (u64)X;
+    q[0].u = p->u_total;
+    q[0].cx = p->cx;
+    q[0].N = X <= p->u_total ? 0 : X / p->u_total;
+    q[0].nc = num_candidates(q[0].N);
+    WindowWork ww;
+    window_work(q, &X, p, p->u_dense, sm_count, ww);
+    for (size_t i = 0; i < ww.items.size() && (int64_t)i < cap; ++i) {
+        out[3 * i] = ww.w[i];
+        out[3 * i + 1] = ww.items[i].b0;
+        out[3 * i + 2] = ww.items[i].b1;
+    }
+    return (int64_t)ww.items.size();
 }
 
 int64_t dr_debug_sieve_plan(int64_t u_total, int64_t u_dense, int32_t segment_log2, int64_t first_wave,

@@ -1050,7 +1050,8 @@ __device__ __forceinline__ int query_of_block(const QueryDev* q, int nq, u64 b) 
 __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const TableView T, u64 n_blocks,
                             u64* __restrict__ ops, u64* __restrict__ acc, i64* __restrict__ counts,
                             S1WinDesc* __restrict__ wdesc, SlotDesc* __restrict__ slots, const S1Band band,
-                            const int mode, TileGroup* __restrict__ tgroups, WinGroup* __restrict__ groups) {
+                            const int mode, TileGroup* __restrict__ tgroups, WinGroup* __restrict__ groups,
+                            u64* __restrict__ near_left) {
     const u64 warps = (u64)gridDim.x * (blockDim.x >> 5);
     const int lane = threadIdx.x & 31;
     for (u64 w = (u64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < 2 * n_blocks; w += warps) {
@@ -1162,6 +1163,10 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
                     }
                 }
                 if (lane == 0) groups[w] = G;
+                if (wc) {
+                    const uint32_t n = __reduce_add_sync(0xffffffffu, near[0] + near[1] + near[2] + near[3]);
+                    if (lane == 0) atomicAdd(reinterpret_cast<uint32_t*>(near_left), n);
+                }
             }
             uint32_t units = 0, rlo = 1, rhi = 0, rend = 0;
             int ngroups = 0;
@@ -1205,10 +1210,11 @@ __global__ void plan_kernel(const QueryDev* __restrict__ qs, int nq, const Table
 
 void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc, i64* counts,
                  S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s, const S1Band& band, int mode,
-                 TileGroup* tgroups, WinGroup* groups) {
+                 TileGroup* tgroups, WinGroup* groups, u64* near_left) {
     if (n_blocks == 0) return;
     const int grid = (int)std::min<u64>((2 * n_blocks + 3) / 4, (u64)sm_count * 16);
-    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode, tgroups, groups);
+    plan_kernel<<<grid, 128, 0, s>>>(q, nq, T, n_blocks, ops, acc, counts, wdesc, slots, band, mode, tgroups, groups,
+                                   near_left);
 }
 
 // Direct answers for queries with X <= table u_total (get_M, :1465-1467).

@@ -166,12 +166,15 @@ constexpr int kCountsPerQuery = 5;
 // A band pass of a streamed table: evaluations with at most this many S1 lookups in the
 // band are summed by the planning thread itself (ops 0 for the sums kernel).
 constexpr int kBandInThread = 64;
+// near_left (with groups): the low word counts the lookups left to the window kernel, which takes
+// off those it sums (both modulo 2^32) -- 0 again when every one of them has been summed.
 // What a planning pass leaves in ops (plan_kernel): work for the sums kernel (every slot),
 // for the tile kernel, or for the sums kernel where the tile kernel takes nothing.
 enum { kPlanSlots = 0, kPlanTiles = 1, kPlanRest = 2 };
 void launch_plan(const QueryDev* q, int nq, const TableView& T, u64 n_blocks, u64* ops, u64* acc,
                  i64* counts, S1WinDesc* wdesc, SlotDesc* slots, int sm_count, cudaStream_t s,
-                 const S1Band& band, int mode, TileGroup* tgroups = nullptr, WinGroup* groups = nullptr);
+                 const S1Band& band, int mode, TileGroup* tgroups = nullptr, WinGroup* groups = nullptr,
+                 u64* near_left = nullptr);
 // Windowed S1 (window length win: a power of two, 2^12 .. 2^16).
 void launch_s1win(const S1WinArgs& a, u64 win, int sm_count, cudaStream_t s);
 int launch_scan_u64(const u64* in, u64* out, u64 n, u64* tmp, size_t tmp_elems, cudaStream_t s);
@@ -196,7 +199,7 @@ struct TileWinArgs {
     const QueryDev* queries;
     TableView T;
     const double* rcp;
-    u64* ticket;
+    u64* ticket;  // [0]: work queue, [1]: the planner's near_left
     u64* acc;
 };
 // The S1 lookups below each block's last window, on the groups of a kPlanTiles pass.

@@ -8,6 +8,9 @@
 // ranges and the one-FMA quotient are those of dr_tiles.cu; the lookups above a block's last
 // window (tile_windows) stay there.  Each lookup is taken by the window q / kTileWin exactly:
 // a block of divisors that reaches past the window, for some member, tests every quotient.
+// Which (window, block) pairs are looked at is the host's choice (window_items), so the planner
+// counts the lookups it leaves to this kernel and the kernel those it sums; a call where they
+// differ fails (a count per lane: sums phase 21.07 -> 21.04 ms at 10^16, 97.85 -> 97.93 at 10^17).
 //
 // Bound: the shared-memory pipe and instruction issue together (1.8 wavefronts per shared
 // load, 8.6 instructions per lookup).  M(10^16): 2.6e10 lookups in 11.8 ms, 2.2e12 a second,
@@ -111,6 +114,7 @@ __global__ void __launch_bounds__(kWinCta, 1024 / kWinCta) windows_kernel(const 
     uint32_t cur_w = 0xFFFFFFFFu;
     int cur_q = -1;
     i64 acc = 0;
+    uint32_t taken = 0;  // lookups summed by this lane's members, modulo 2^32
     for (;;) {
         __syncthreads();  // every warp is done with the task before and its window
         if (threadIdx.x == 0) {
@@ -206,6 +210,7 @@ __global__ void __launch_bounds__(kWinCta, 1024 / kWinCta) windows_kernel(const 
                 if (umin > umax) continue;
                 res = __reduce_max_sync(0xffffffffu, member && cnt > 0 ? res : 0u);
                 const uint32_t tot = __reduce_add_sync(0xffffffffu, some ? (uint32_t)hi - lo + 1u : 0u);
+                if (mine == 0 && some) taken += (uint32_t)hi - lo + 1u;
                 const int sgn = ((dbits >> 2) & 1u) == ((dbits >> (5 + 3 * g)) & 1u) ? 1 : -1;
                 if (umax - umin < kNarrow) {
                     // few divisors, all members at once: lanes on members, the divisors in turn
@@ -250,7 +255,10 @@ __global__ void __launch_bounds__(kWinCta, 1024 / kWinCta) windows_kernel(const 
                         else acc += win_block<true>(base, E, R, r, i0, ma, mb, lane);
                     }
                 } else {
-                    // few members at a time: one after another
+                    // few members at a time: one after another.  `part` fits 32 bits: `parts` is
+                    // cut so that a unit holds about 131072 lookups by the estimate of window_items,
+                    // which is never below one member's share, and where it stops at 1024 pieces a
+                    // lane's share of the divisors, below 2^31, is at most 2^16 of |M| < 27000.
                     unsigned left = __ballot_sync(0xffffffffu, some);
                     while (left) {
                         const int m = __popc(mm & ((left & -left) - 1u));
@@ -279,6 +287,8 @@ __global__ void __launch_bounds__(kWinCta, 1024 / kWinCta) windows_kernel(const 
         const u64 t = warp_sum_u64((u64)acc);
         if (lane == 0) atomicAdd(a.acc + 3 * cur_q + 1, t);
     }
+    taken = __reduce_add_sync(0xffffffffu, taken);
+    if (lane == 0) atomicAdd(reinterpret_cast<uint32_t*>(a.ticket + 1), 0u - taken);
 }
 
 static_assert(offsetof(WinShared, win) % 16 == 0 && kTileWin % 8 == 0, "16-byte staging copies");

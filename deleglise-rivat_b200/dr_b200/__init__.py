@@ -160,6 +160,7 @@ def lib():
                                   ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float)]),
             "dr_mlp_train": (i32, [vp, ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float), i64, i32,
                                    ctypes.c_float, ctypes.POINTER(ctypes.c_float)]),
+            "dr_debug_window_items": (i64, [i64, P, i32, ctypes.POINTER(i64), i64]),
             "dr_debug_mlp_train_steps": (i32, [vp, ctypes.POINTER(ctypes.c_float), ctypes.POINTER(ctypes.c_float), i64,
                                                i32, ctypes.c_float, ctypes.POINTER(ctypes.c_float)]),
             "dr_tuner_features": (i32, [i64, u64, i32, i32, ctypes.POINTER(ctypes.c_float)]),
@@ -190,6 +191,7 @@ def exported_symbols() -> list:
         "dr_mlp_create", "dr_mlp_destroy", "dr_mlp_num_params", "dr_mlp_set_weights", "dr_mlp_get_weights",
         "dr_mlp_forward", "dr_mlp_grad", "dr_mlp_train", "dr_tuner_features", "dr_tuner_params", "dr_tuner_propose",
         "dr_measure_peaks", "dr_debug_sieve_plan", "dr_debug_stream_plan", "dr_debug_mlp_train_steps",
+        "dr_debug_window_items",
     ]
 
 
@@ -220,6 +222,17 @@ def stream_plan(u_total: int, u_dense: int, segment_log2: int, u_resident: int, 
     buf = (ctypes.c_int64 * (3 * max(n, 1)))()
     lib().dr_debug_stream_plan(*args, buf, n)
     return ures.value, [(buf[3 * i], buf[3 * i + 1], bool(buf[3 * i + 2])) for i in range(n)]
+
+
+def window_items(X: int, params: Params, sm_count: int = 148) -> list:
+    """The window kernel's items for M(X) on its own table: (window, first block, end block)."""
+    args = (int(X), ctypes.byref(params), int(sm_count))
+    n = int(lib().dr_debug_window_items(*args, None, 0))
+    if n < 0:
+        _check(n)
+    buf = (ctypes.c_int64 * (3 * max(n, 1)))()
+    lib().dr_debug_window_items(*args, buf, n)
+    return [(buf[3 * i], buf[3 * i + 1], buf[3 * i + 2]) for i in range(n)]
 
 
 def measure_peaks(device: int = 0) -> dict:

@@ -226,6 +226,11 @@ int64_t dr_debug_sieve_plan(int64_t u_total, int64_t u_dense, int32_t segment_lo
  * count (0: nothing streams) or a negative DR_ERR_* code.  Needs no GPU. */
 int64_t dr_debug_stream_plan(int64_t u_total, int64_t u_dense, int32_t segment_log2, int64_t u_resident,
                              int64_t band_values, int64_t *u_res, int64_t *out, int64_t cap);
+/* The window kernel's work for one M(X) on a table of its own (p) -- test support, no
+ * counterpart in the reference: per item {w, b0, b1}, the blocks [b0, b1) of 32 candidates
+ * coprime to 6 whose S1 lookups with quotients in window w (98304 values) it sums.  Writes
+ * at most cap triples; returns the item count or a negative DR_ERR_* code.  Needs no GPU. */
+int64_t dr_debug_window_items(int64_t X, const dr_params *p, int32_t sm_count, int64_t *out, int64_t cap);
 /* dr_mlp_train by its step-by-step route on any device -- test support, no counterpart in
  * the reference: the same weights and loss, bit for bit. */
 int dr_debug_mlp_train_steps(dr_mlp *mlp, const float *x, const float *t, int64_t B, int steps, float lr,
