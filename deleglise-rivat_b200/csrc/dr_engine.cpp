@@ -45,9 +45,13 @@ int fail(int code, const char* fmt, ...) {
     } while (0)
 
 // Sieving primes up to which squares are not bucketed: the buckets' five launches take about
-// 20 us, the squares in the sieve itself less up to about 1.5e9 values (1e6 values 0.046 ->
-// 0.024 ms, 1e9 0.948 -> 0.919 ms; 2e9 the same, 5.4e9 4.42 -> 4.50 ms).
-constexpr size_t kBucketMinPrimes = 4096;
+// 20 us, the squares in the sieve itself less up to about 1.5e9 values with 1024 threads (1e6
+// values 0.046 -> 0.024 ms, 1e9 0.948 -> 0.919 ms; 2e9 the same, 5.4e9 4.42 -> 4.50 ms).  With
+// fewer threads each takes more of the primes in every segment and the sizes that break even
+// are smaller (buckets -> none: 512 threads 2^18 8e8 0.943 -> 0.938 ms, 1.4e9 1.606 -> 1.641; 256
+// threads 2^15 4e8 0.573 -> 0.558, 1.4e9 1.938 -> 2.120; 128 threads 2^15 4e8 0.562 -> 0.558, 1e9
+// 1.330 -> 1.436).
+size_t bucket_min_primes(int block) { return 2048 + 2 * (size_t)block; }
 // The window kernel takes S1 lookups where a launch has this many of them, from queries of at
 // least kWinMinX (sums phase without -> with it: X = 10^14 1.37 -> 1.58 ms, 10^14.5 2.83 -> 2.59
 // ms at about 2.4e9 lookups, 10^15 5.3 -> 4.8, 10^16 25.9 -> 21.6, 10^17 136 -> 101 ms).
@@ -486,7 +490,7 @@ int build_table(dr_ctx* c, int64_t u_total, int64_t u_dense, int64_t mu_limit, c
     a.sq_seg0 = 0;
     a.sq_pos = nullptr;
     // few primes: their squares are marked by the sieve, a prime per thread
-    if (pr.size() <= kBucketMinPrimes) sq_hits = 0;
+    if (pr.size() <= bucket_min_primes(block)) sq_hits = 0;
     if (sq_hits == 0) a.sqC_first = (int)pr.size();
     if (sq_hits > 0) {
         if ((rc = ensure(c, c->sq_cnt, (size_t)nseg * 8))) return rc;
