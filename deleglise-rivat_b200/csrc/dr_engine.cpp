@@ -57,6 +57,12 @@ size_t bucket_min_primes(int block) { return 2048 + 2 * (size_t)block; }
 // ms at about 2.4e9 lookups, 10^15 5.3 -> 4.8, 10^16 25.9 -> 21.6, 10^17 136 -> 101 ms).
 constexpr double kWinMinLookups = 2e9;
 constexpr int64_t kWinMinX = 1000000000000LL;
+// ... and of split parameters from kWinMinCx on.  Below, most divisors lie far above sqrt(y),
+// where 32 neighbours' quotients share one line of the table and the tile kernel reads them as
+// fast, while one block of the first candidates holds more of a window than a CTA should (sums
+// phase with -> without windows: cx = 0.05, X = 10^13, u = 10^9 41.7 -> 1.6 ms, 0.1, 10^15, 10^10
+// 47.1 -> 21.6, 0.2, 10^14, 10^9 8.07 -> 3.68; 0.3, 10^15, 10^10 8.53 -> 9.06, 0.6 5.07 -> 5.86).
+constexpr double kWinMinCx = 0.3;
 constexpr int64_t kDenseInt16Limit = 7600000000LL;  // |M(n)| < 32768 for n <= 7.6e9
 
 struct DevBuf {
@@ -964,7 +970,7 @@ int stream_bands(dr_ctx* c, const StreamPlan& sp, const SumsArgs& base, int grid
 // tier and below 2^31; none where the query is too small to gain from them.  A window at q
 // holds about X W / (2 q^2) lookups in all; one with fewer than 2^18 is not worth its staging.
 u64 window_limit(int64_t X, const dr_params& p, int64_t u_dense) {
-    if (X <= p.u_total || p.u_total < 1 || X < kWinMinX) return 0;
+    if (X <= p.u_total || p.u_total < 1 || X < kWinMinX || p.cx < kWinMinCx) return 0;
     const double q = std::sqrt((double)X * (double)kTileWin / (2.0 * 262144.0));
     return (u64)(std::min(q, (double)std::min<int64_t>(u_dense, (int64_t(1) << 31) - 1)) / (double)kTileWin);
 }
@@ -1025,7 +1031,7 @@ void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P
                  WindowWork& out) {
     double total = 0.0;
     for (size_t i = 0; i < qs.size(); ++i)
-        if (qs[i].N > 0 && X[i] >= kWinMinX)
+        if (qs[i].N > 0 && X[i] >= kWinMinX && P[i].cx >= kWinMinCx)
             total += 0.53 * std::sqrt((double)X[i] * (double)qs[i].N) / P[i].cx;  // S1 lookups, about
     if (total < kWinMinLookups) return;
     const double task = std::max(total / (sm_count * 12.0), 524288.0);  // a dozen to a CTA

@@ -5,7 +5,9 @@ whose quotient lies in the first tile_windows(block) windows of 98304 values; th
 name, per window, the blocks that the window kernel looks at.  They must be the blocks whose
 windows include it, less leading ones whose smallest quotient lies above the window: that
 quotient is worked out here from the split point as the planner does.  Split parameters over
-the whole accepted range, far from the defaults above all."""
+the whole range that takes windows, far from the defaults above all.  Below 0.3 there are none:
+long divisor ranges read the table as fast from the tile kernel, and one block of the first
+candidates would hold a window's work for one CTA."""
 import math
 import random
 
@@ -36,7 +38,6 @@ def _smallest_quotient(y, cx):
 
 
 CASES = [(X, cx, u) for cx, sizes in (
-    (0.01, ((10**13, 10**9), (10**15, 10**12))), (0.03, ((10**13, 10**9), (2 * 10**15, 4 * 10**10))),
     (0.3, ((10**14, 10**9), (10**16, 5 * 10**9))), (1.25, ((10**15, 5 * 10**9), (10**17, 10**11))),
     (6.0, ((10**15, 3 * 10**8), (10**17, 3 * 10**9))), (17.0, ((2 * 10**15, 8 * 10**8), (10**17, 6 * 10**9))),
     (40.0, ((10**16, 4 * 10**9), (10**17, 1.3 * 10**10))), (63.0, ((10**17, 2 * 10**10),))) for X, u in sizes]
@@ -77,3 +78,10 @@ def test_items_cover_the_near_lookups(X, cx, u):
             for k in [last] + [rng.randrange(1, last + 1) for _ in range(20)]:
                 for y in (X // k,) + ((X // k // 3,) if 3 * k <= N else ()):
                     assert _smallest_quotient(y, cx) >= (w + 1) * W, (w, k)
+
+
+@pytest.mark.parametrize("X,cx,u", [(10**13, 0.01, 10**9), (10**13, 0.05, 10**9), (10**15, 0.1, 10**10),
+                                    (10**14, 0.2, 10**9), (2 * 10**15, 0.2999, 10**10)])
+def test_no_windows_for_long_ranges(X, cx, u):
+    p = dr_b200.Params(u_total=u, u_dense=u // 8, cx=cx, mu_limit=u)
+    assert dr_b200.window_items(X, p) == []
