@@ -1073,6 +1073,34 @@ void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P
     out.tasks = std::move(sorted);
 }
 
+// Whether the tile kernel or the sums kernel takes a launch's evaluations.  The tile kernel's
+// time per term falls with the candidates that share a block of divisors: about 0.35 of the sums
+// kernel's where all 32 do, several times it for the first blocks, whose members' ranges hardly
+// meet.  Against the sums kernel that is 0.35 + 0.65 sqrt(t / N), with t, where the two meet, 100 at
+// u = 2e7 and growing as u^0.33 with the table.  A launch of little work also waits for its longest
+// units: the gain has to make up for `wait` terms.  Sums phase, sums / tile kernel, ms:
+//   300 queries, u = 2e7   N = 30 0.15 / 0.27, 100 0.38 / 0.37, 300 0.80 / 0.63
+//   300 queries, u = 5e8   N = 30 0.34 / 0.64, 200 1.43 / 1.86, 400 2.53 / 2.66, 1000 5.75 / 4.77
+//   30 queries, u = 2e7    N = 30 0.067 / 0.145, 400 0.188 / 0.206, 1000 0.383 / 0.233
+//   one query, u = 2e7     N = 300 0.059 / 0.087, 3000 0.081 / 0.101, 10000 0.146 / 0.125
+//   one query, u = 5e8     N = 1000 0.083 / 0.158, 3000 0.150 / 0.194, 10000 0.324 / 0.262
+//   100 queries, u = 1e10  N = 100 0.96 / 1.59, 300 2.56 / 3.04, 1000 7.62 / 7.39
+// Tables below 10^6 values, and a handful of candidates (16 slots), lose nothing on tiles that the
+// noise would not hide (u = 3e3, N = 102 0.188 / 0.054; u = 4.5e5, N = 2200 0.070 / 0.075).
+bool tiles_pay(const std::vector<QueryDev>& qs, u64 slots) {
+    if (slots <= 16) return true;
+    double gain = 0.0, work = 0.0, wait = 0.0;  // wait: weighted by work
+    for (const QueryDev& q : qs) {
+        if (q.nc == 0) continue;
+        const double u = (double)q.u, r = std::sqrt(u), t = 100.0 * std::pow(u / 2e7, 0.33);
+        const double terms = std::sqrt((double)q.X * (double)q.N) * (0.57 / q.cx + 0.27 * q.cx);
+        work += terms;
+        gain += terms * (1.0 - std::sqrt(t / (double)q.N));
+        if (u >= 1e6) wait += terms * std::min(std::min(1.5 * u, 4500.0 * r), std::max(1e8, 2000.0 * r));
+    }
+    return gain * work > wait;
+}
+
 // Room for n op counts, their prefix and the scan's scratch.
 int reserve_ops(dr_ctx* c, u64 n) {
     int rc = ensure(c, c->ops, (size_t)std::max<u64>(n, 1) * 8);
@@ -1176,7 +1204,8 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     // beside them, ops per slot and the sums kernel for everything: a block holds up to 64 slots
     // (16 bytes each; 352 for the records and the ops of the block), so only calls that need the
     // ops per slot anyway, or whose queries have a few candidates each, come to that.
-    bool tiles = witems.empty();  // the windowed S1 leaves every other lookup to the sums kernel
+    // the windowed S1 leaves every other lookup to the sums kernel
+    bool tiles = witems.empty() && tiles_pay(qs, slots);
     const bool per_slot = !tiles || sp || rest;
     if ((rc = reserve_ops(c, per_slot ? slots : 2 * blocks))) return rc;
     if (tiles && ensure(c, c->tgroups, (size_t)std::max<u64>(2 * blocks, 1) * sizeof(TileGroup))) {
