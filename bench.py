@@ -254,13 +254,13 @@ def sieve_marks(u_total, u_dense, sm_count, S=1 << 17):
 
 # Warp instructions per unit of work, from ncu smsp__inst_executed.sum of one launch
 # divided by that launch's work:
-#   S1/S2 phase at M(10^16) (B200 policy), tile and window kernels: the S2 positions
-#     (timing-only build that keeps only them) 4.95e9 instructions for 1.12e10 positions,
-#     the S1 lookups (window kernel, and the tile kernel without S2) 7.05e9 for 2.79e10;
-#   sieve_kernel, odd mode, on the M(10^15) table: 5.63e7 instructions for 1.01e8 values.
-SUMS_INST_PER_S1 = 0.253
+#   S1/S2 phase at M(10^16) (B200 policy): window kernel 6.97e9 and tile kernel 5.08e9
+#     instructions for 2.79e10 S1 lookups and 1.12e10 S2 positions; the positions 4.95e9 (the
+#     tile kernel in a timing-only build without S1), the lookups the rest;
+#   sieve_kernel, odd mode, on the M(10^15) table: 5.17e7 instructions for 1.01e8 values.
+SUMS_INST_PER_S1 = 0.254
 SUMS_INST_PER_S2 = 0.442
-SIEVE_INST_PER_VALUE = 0.556
+SIEVE_INST_PER_VALUE = 0.511
 # DRAM bytes per op of the S1/S2 phase (dram__bytes_read.sum + dram__bytes_write.sum of the
 # tile and the window kernel over S1 lookups + S2 positions) at M(10^15): 8.25 GB / 7.80e9 ops.
 SUMS_DRAM_PER_OP = 1.06

@@ -701,7 +701,7 @@ __device__ __forceinline__ void tile_range(const SlotDesc& t, int g, uint32_t* l
 }
 
 // Work units of segment g over the index range [ulo, uhi]; S2 blocks start on a multiple of
-// 32 positions (one Mobius word per warp load).  An S1 block counts kTileS1Units: its gathers
+// 32 positions (aligned 512-byte warp reads of invw).  An S1 block counts kTileS1Units: its gathers
 // take that much longer than an S2 block.
 __device__ __forceinline__ uint32_t tile_units(int g, uint32_t ulo, uint32_t uhi) {
     if (ulo > uhi) return 0;

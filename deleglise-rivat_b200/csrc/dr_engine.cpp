@@ -768,9 +768,10 @@ bool band_odd(const StreamPlan& sp, int64_t vlo, int64_t vhi) {
     return sp.u_dense % 64 == 0 && vlo >= 2 * sp.u_dense && vhi + 2 * (int64_t)sp.S <= 2 * sp.u_res;
 }
 
-// Decide whether the query streams, and reserve every buffer the bands use before the
-// resident build (nothing may grow once launches are queued: the segment offsets of the
-// resident table carry into the first band).  *sp.nbands == 0: no streaming.
+// Decide whether the query streams, and reserve every buffer that the bands share with the
+// resident build before it (it leaves them its segment offsets, and a buffer that grows loses
+// what it holds); the query buffers and the kept plane words hold nothing of it and are
+// reserved later.  *sp.nbands == 0: no streaming.
 int plan_stream(dr_ctx* c, int64_t X, int64_t ut, int64_t ud, int64_t ml, const dr_params& tune, StreamPlan* sp) {
     int S0, block;
     pick_shape(ut, &tune, &S0, &block);
@@ -1667,7 +1668,9 @@ uint64_t dr_query_bytes(int64_t X, const dr_params* p) {
     uint64_t b = dr_table_bytes(p->u_total, p->u_dense, p->mu_limit);
     if (X > p->u_total && p->cx > 0.0) {
         const double inv = 1.4143 * std::sqrt((double)X) / p->cx + 65.0;  // S1 reciprocals
-        const int64_t slots = 2 * num_candidates(X / p->u_total);        // ops + prefix
+        // ops, prefix and record of every evaluation: the sums kernel's form, which no call
+        // exceeds that cannot (the tile kernel's takes less, or is given up)
+        const int64_t slots = 2 * num_candidates(X / p->u_total);
         b += (uint64_t)(8.0 * inv) + (uint64_t)(p->mu_limit / 6 + 1) * 16 + (uint64_t)slots * (16 + sizeof(SlotDesc)) +
              scan_u64_tmp_elems((u64)slots) * 8;
     }

@@ -22,6 +22,8 @@
 // (dense table).  Two CTAs of 8 warps per SM (128 registers, no spills) beat three (80) and
 // four (64): 28.9, 29.0, 31.5 ms at M(10^16).
 //
+// Launches of little work or of few candidates stay with the sums kernel (tiles_pay, dr_engine.cpp).
+//
 // Sums: mertens_dr.hpp:1490-1614 (S1), :462-660 (S2).
 #include "dr_kernels.cuh"
 

@@ -13,7 +13,7 @@
 // differ fails (a count per lane: sums phase 21.07 -> 21.04 ms at 10^16, 97.85 -> 97.93 at 10^17).
 //
 // Bound: the shared-memory pipe and instruction issue together (1.8 wavefronts per shared
-// load, 8.6 instructions per lookup).  M(10^16): 2.6e10 lookups in 11.8 ms, 2.2e12 a second,
+// load, 8.6 instructions per lookup).  M(10^16): 2.6e10 lookups in 11.4 ms, 2.3e12 a second,
 // against 0.26e12 (no two lanes on one line) to 2.4e12 from global memory; the sums phase as a
 // whole 25.9 -> 21.6 ms, at 10^17 136 -> 101 ms.  Windows of 98304 values by one CTA of 32
 // warps; 49152 by two of 16: 22.7 and 112 ms.
