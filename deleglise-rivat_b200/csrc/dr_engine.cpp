@@ -1074,32 +1074,43 @@ void window_work(std::vector<QueryDev>& qs, const int64_t* X, const dr_params* P
     out.tasks = std::move(sorted);
 }
 
-// Whether the tile kernel or the sums kernel takes a launch's evaluations.  The tile kernel's
-// time per term falls with the candidates that share a block of divisors: about 0.35 of the sums
-// kernel's where all 32 do, several times it for the first blocks, whose members' ranges hardly
-// meet.  Against the sums kernel that is 0.35 + 0.65 sqrt(t / N), with t, where the two meet, 100 at
-// u = 2e7 and growing as u^0.33 with the table.  A launch of little work also waits for its longest
-// units: the gain has to make up for `wait` terms.  Sums phase, sums / tile kernel, ms:
+// Whether the tile kernel or the sums kernel takes a launch's evaluations: the smaller of two
+// estimates of the phase, in microseconds, fitted to both kernels' times on 1374 launches (1 to 400
+// queries, u from 3e3 to 1e10, N = X/u up to 8e5, cx from 0.02 to 25; median error 15%; the choice
+// costs 1.5% over the better kernel's time on average; with tiles alone 397 of them were slower than
+// before the tile kernel, with the choice 6, by up to 1.23).  The tile kernel pays for the blocks of divisors that a group's members span
+// together -- with few candidates the first blocks, whose members' ranges hardly meet, are most of
+// the work -- and waits for its longest units where there are fewer blocks than warps; the sums
+// kernel pays five times as much a term.  Sums kernel / tile kernel, ms:
 //   300 queries, u = 2e7   N = 30 0.15 / 0.27, 100 0.38 / 0.37, 300 0.80 / 0.63
 //   300 queries, u = 5e8   N = 30 0.34 / 0.64, 200 1.43 / 1.86, 400 2.53 / 2.66, 1000 5.75 / 4.77
-//   30 queries, u = 2e7    N = 30 0.067 / 0.145, 400 0.188 / 0.206, 1000 0.383 / 0.233
 //   one query, u = 2e7     N = 300 0.059 / 0.087, 3000 0.081 / 0.101, 10000 0.146 / 0.125
 //   one query, u = 5e8     N = 1000 0.083 / 0.158, 3000 0.150 / 0.194, 10000 0.324 / 0.262
 //   100 queries, u = 1e10  N = 100 0.96 / 1.59, 300 2.56 / 3.04, 1000 7.62 / 7.39
-// Tables below 10^6 values, and a handful of candidates (16 slots), lose nothing on tiles that the
-// noise would not hide (u = 3e3, N = 102 0.188 / 0.054; u = 4.5e5, N = 2200 0.070 / 0.075).
-bool tiles_pay(const std::vector<QueryDev>& qs, u64 slots) {
-    if (slots <= 16) return true;
-    double gain = 0.0, work = 0.0, wait = 0.0;  // wait: weighted by work
+// Queries of few candidates (N below about 300 on average over the work, 3e6 terms or more) are where
+// the estimate of the tile kernel falls short, and it has to win by 15% there.
+// Below 6e5 terms the sums kernel's chunks are too few and the tile kernel is the better one
+// (u = 3e3, N = 102 0.188 / 0.054).
+bool tiles_pay(const std::vector<QueryDev>& qs) {
+    double s1 = 0.0, s2 = 0.0, span = 0.0, blocks = 0.0, cands = 0.0, members = 0.0, few = 0.0;
     for (const QueryDev& q : qs) {
         if (q.nc == 0) continue;
-        const double u = (double)q.u, r = std::sqrt(u), t = 100.0 * std::pow(u / 2e7, 0.33);
-        const double terms = std::sqrt((double)q.X * (double)q.N) * (0.57 / q.cx + 0.27 * q.cx);
-        work += terms;
-        gain += terms * (1.0 - std::sqrt(t / (double)q.N));
-        if (u >= 1e6) wait += terms * std::min(std::min(1.5 * u, 4500.0 * r), std::max(1e8, 2000.0 * r));
+        const double rx = std::sqrt((double)q.X), rn = std::sqrt((double)q.N), nb = (double)((q.nc + 31) / 32);
+        s1 += 0.57 * rx * rn / q.cx;  // S1 lookups and S2 positions, about
+        s2 += 0.27 * rx * rn * q.cx;
+        few += rx * (0.57 / q.cx + 0.27 * q.cx);  // terms / sqrt(N)
+        // units' blocks: the ranges of candidates 1, 97, 193, ..., every other S1 divisor in 128s,
+        // S2 positions in 64s
+        span += (nb > 1.0 ? 1.0 + 0.204 * (std::sqrt(nb) - 0.75) : 1.0) * rx * (1.0 / (256.0 * q.cx) + q.cx / 768.0);
+        blocks += nb;
+        cands += (double)q.nc;
+        members = std::max(members, std::min((double)q.nc, 32.0));
     }
-    return gain * work > wait;
+    if (s1 + s2 < 6e5) return true;
+    const double tiles = 51.0 + 2.0e-3 * span + 1.6e-7 * s1 + 2.3e-7 * s2 + 0.039 * blocks +
+                         std::min(span / 2368.0, 1.0) * (18.0 + 1.55 * members);
+    const double sums = 62.0 + 9.2e-7 * s1 + 1.1e-6 * s2 + 6.4e-3 * cands + 32.0 * std::min(cands / 2000.0, 1.0);
+    return tiles < (s1 + s2 > 3e6 && few * std::sqrt(300.0) > s1 + s2 ? 0.85 : 1.02) * sums;
 }
 
 // Room for n op counts, their prefix and the scan's scratch.
@@ -1206,7 +1217,7 @@ int enqueue_queries(dr_ctx* c, const int64_t* X, const dr_params* P, int64_t nq,
     // (16 bytes each; 352 for the records and the ops of the block), so only calls that need the
     // ops per slot anyway, or whose queries have a few candidates each, come to that.
     // the windowed S1 leaves every other lookup to the sums kernel
-    bool tiles = witems.empty() && tiles_pay(qs, slots);
+    bool tiles = witems.empty() && tiles_pay(qs);
     const bool per_slot = !tiles || sp || rest;
     if ((rc = reserve_ops(c, per_slot ? slots : 2 * blocks))) return rc;
     if (tiles && ensure(c, c->tgroups, (size_t)std::max<u64>(2 * blocks, 1) * sizeof(TileGroup))) {

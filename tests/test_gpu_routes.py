@@ -23,9 +23,9 @@ def _kernels(call):
 
 
 @pytest.mark.parametrize("count,u,N,takes", [
-    (1, 10**5, 5, "tiles_kernel"), (1, 10**5, 1000, "tiles_kernel"), (1, 2 * 10**7, 300, "sums_kernel"),
+    (1, 10**5, 5, "tiles_kernel"), (1, 10**5, 1000, "tiles_kernel"), (1, 5 * 10**8, 1000, "sums_kernel"),
     (1, 2 * 10**7, 20000, "tiles_kernel"), (300, 2 * 10**7, 30, "sums_kernel"), (300, 2 * 10**7, 600, "tiles_kernel"),
-    (300, 5 * 10**8, 30, "sums_kernel"), (300, 5 * 10**8, 1000, "tiles_kernel"), (40, 10**6, 4, "sums_kernel")])
+    (300, 5 * 10**8, 30, "sums_kernel"), (300, 5 * 10**8, 1000, "tiles_kernel"), (40, 10**6, 4, "tiles_kernel")])
 def test_route(engine, count, u, N, takes):
     X, cx = u * N + u // 2, 1.25
     xs = [X + 7 * k for k in range(count)]
